@@ -64,11 +64,12 @@ struct pic_ctx {
   long long*                                      jfix       = nullptr;
   size_t                                          jfix_elems = 0;
   unsigned*                                       jfix_bound = nullptr;
-  // deposit records of the tiled kernel (FP32; allocated on first use):
-  // stage_slots buffers and their claim words (sizes: run_tiled)
+  // deposit records of the tiled kernel (allocated on first use): stage_slots
+  // buffers and their claim words
   uint4*                                          stage_rec   = nullptr;
   unsigned*                                       stage_claim = nullptr;
   int                                             stage_slots = 0;
+  bool                                            stage_tried = false;
 };
 
 namespace pic_internal {

@@ -220,42 +220,57 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
   a.err        = c->d_err;
   const int D = c->grid.dim, O = c->grid.order;
   {
-    // lanes of a warp over about four cells: the stride from the species'
-    // mean particles per cell
+    // 2D: the lanes of a warp spread over about four cells, the stride from the
+    // species' mean particles per cell (they deposit as they are pushed). 3D:
+    // consecutive particles (their deposit is ordered by its records, and the
+    // field reads of one cell broadcast). Strides 1, 2 and 4 took 13.4, 13.7
+    // and 14.3 ms per step of the 96^3 sweep plasma, 0.998, 1.040 and 1.108 ms
+    // of 100 x 75 x 61 turbulence, 0.447, 0.424 and 0.431 ms of the 512^2 pair
+    // plasma (16 ppc)
     int64_t np = 0, cells = 1;
     for (int k = 0; k < a.nsp; ++k) np += sps[k]->npart;
     for (int d = 0; d < D; ++d) cells *= c->grid.n[d];
     const int64_t ppc = np / std::max<int64_t>(1, (int64_t)a.nsp * cells);
-    a.lane_stride     = ppc >= 24 ? 4 : (ppc >= 12 ? 2 : 1);
+    a.lane_stride     = D == 3 || ppc < 12 ? 1 : (ppc >= 24 ? 4 : 2);
   }
-  if (sizeof(real) == 4 && O >= 1 && (D == 3 || O <= 2)) {
-    // 3D: two buffers per SM (one CTA per SM); 2D: eight smaller ones (up to
-    // five CTAs per SM). The launcher checks them against the kernel's
-    // occupancy and deposits directly when they do not suffice.
-    const int cap = D == 2 ? pic::kStageCap / 4 : (O == 3 ? 2 * pic::kStageCap : pic::kStageCap);
-    if (!c->stage_rec) {
-      const int n = (D == 2 ? 8 : 2) * pic::sm_count();
-      if (cudaMalloc((void**)&c->stage_rec, sizeof(uint4) * 2 * (size_t)cap * n) !=
-              cudaSuccess ||
-          cudaMalloc((void**)&c->stage_claim, sizeof(unsigned) * (size_t)n) != cudaSuccess ||
-          cudaMemsetAsync(c->stage_claim, 0, sizeof(unsigned) * (size_t)n, s) != cudaSuccess) {
+  cudaError_t e = cudaErrorInvalidValue;
+  if (!c->stage_tried) {
+    // the deposit records' buffers, once per context (its dimension, order
+    // and precision fix their size); without them every particle deposits as
+    // it is pushed
+    size_t words = 0;
+    int    slots = 0;
+#define PIC_RW(DD, OO) \
+  if (D == DD && O == OO) e = pic::deposit_record_words<DD, OO, real>(&words, &slots);
+    PIC_RW(2, 0)
+    PIC_RW(2, 1)
+    PIC_RW(2, 2)
+    PIC_RW(2, 3)
+    PIC_RW(3, 0)
+    PIC_RW(3, 1)
+    PIC_RW(3, 2)
+    PIC_RW(3, 3)
+#undef PIC_RW
+    if (e != cudaSuccess) return PIC_ERR_CUDA;
+    if (slots > 0) {
+      if (cudaMalloc((void**)&c->stage_rec, sizeof(uint4) * words * (size_t)slots) != cudaSuccess ||
+          cudaMalloc((void**)&c->stage_claim, sizeof(unsigned) * (size_t)slots) != cudaSuccess ||
+          cudaMemsetAsync(c->stage_claim, 0, sizeof(unsigned) * (size_t)slots, s) != cudaSuccess) {
         cudaGetLastError();
         if (c->stage_rec) cudaFree(c->stage_rec);
         if (c->stage_claim) cudaFree(c->stage_claim);
         c->stage_rec   = nullptr;
         c->stage_claim = nullptr;
       } else {
-        c->stage_slots = n;
+        c->stage_slots = slots;
       }
     }
-    if (c->stage_rec) {
-      a.st.rec    = c->stage_rec;
-      a.st.claim  = c->stage_claim;
-      a.st.nslots = c->stage_slots;
-      a.st.cap    = cap;
-    }
+    c->stage_tried = true;
   }
-  cudaError_t e = cudaErrorInvalidValue;
+  a.st.rec    = c->stage_rec;
+  a.st.claim  = c->stage_claim;
+  a.st.nslots = c->stage_slots;
+  e           = cudaErrorInvalidValue;
 #define PIC_TD(DD, OO) \
   if (D == DD && O == OO) e = pic::launch_push_deposit_tiled<DD, OO, real>(a, s);
   PIC_TD(2, 0)

@@ -4,11 +4,12 @@
 // deposit. Every routine follows the operation order of the reference kernel
 // it cites (paths relative to the entity repository) so that, compiled with
 // -fmad=false, a particle's new cell, offset and momentum are bit-identical to
-// the reference arithmetic; the one deliberate contraction is the running sum
-// of the field interpolation at order >= 1, written as an explicit fma.
+// the reference arithmetic (but for the sign of an exactly zero field). The
+// deposit has two forms, the reference's expressions and a factored one.
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "pic_types.h"
@@ -50,14 +51,19 @@ __device__ __forceinline__ int stag_of(int c, int a) {
 // shape functions: src/kernels/particle_shapes.hpp:25-63, 544-614
 // ---------------------------------------------------------------------------
 template <typename real>
+__device__ __forceinline__ real S3near(real x) {
+  const real HALF = 0.5;
+  return (real)(2.0 / 3.0) - x * x + HALF * (x * x * x);
+}
+template <typename real>
+__device__ __forceinline__ real S3far(real x) {
+  const real TWO = 2;
+  return (real)(4.0 / 3.0) - TWO * x + x * x - (real)(1.0 / 6.0) * (x * x * x);
+}
+template <typename real>
 __device__ __forceinline__ real S3f(real x) {
-  const real ONE = 1, TWO = 2, HALF = 0.5;
-  if (x < ONE) {
-    return (real)(2.0 / 3.0) - x * x + HALF * (x * x * x);
-  } else if (x < TWO) {
-    return (real)(4.0 / 3.0) - TWO * x + x * x - (real)(1.0 / 6.0) * (x * x * x);
-  }
-  return (real)0;
+  const real ONE = 1, TWO = 2;
+  return x < ONE ? S3near(x) : (x < TWO ? S3far(x) : (real)0);
 }
 
 template <int O, bool STAG, typename real>
@@ -100,20 +106,23 @@ __device__ __forceinline__ void shape(int i, real di, int& imin, real* S) {
     }
   } else {
     static_assert(O == 3, "shape orders 1..3");
-    if constexpr (!STAG) {
-      imin = i - 1;
-#pragma unroll
-      for (int n = 0; n < 4; n++) S[n] = S3f<real>(fabs(ONE + di - (real)n));
+    // |t - n| is the distance to node n; for 1 < t < 2 its pieces are known
+    // (t and 3 - t in (1, 2), t - 1 and 2 - t in (0, 1)): one test in place of
+    // two per node
+    real t = ONE + di;
+    imin   = i - 1;
+    if constexpr (STAG) {
+      t = (di < HALF ? (real)1.5 : HALF) + di;
+      if (di < HALF) imin = i - 2;
+    }
+    if (t > ONE && t < (real)2) {
+      S[0] = S3far<real>(t);
+      S[1] = S3near<real>(t - ONE);
+      S[2] = S3near<real>((real)2 - t);
+      S[3] = S3far<real>((real)3 - t);
     } else {
-      if (di < HALF) {
-        imin = i - 2;
 #pragma unroll
-        for (int n = 0; n < 4; n++) S[n] = S3f<real>(fabs((real)1.5 + di - (real)n));
-      } else {
-        imin = i - 1;
-#pragma unroll
-        for (int n = 0; n < 4; n++) S[n] = S3f<real>(fabs(HALF + di - (real)n));
-      }
+      for (int n = 0; n < 4; n++) S[n] = S3f<real>(fabs(t - (real)n));
     }
   }
 }
@@ -295,51 +304,120 @@ __device__ __forceinline__ void interp_zigzag(const V& EB, const int* ic,
   }
 }
 
+// Two floats in one 64-bit register: the packed operations round each half
+// as the scalar ones do and take one issue slot for both. The assembler
+// contracts a packed product and sum into one multiply-add, whatever
+// -fmad=false says (it leaves scalar ones alone), so a sum is written as
+// x * 1 + y with a one it cannot see through; the parity tests would show a
+// contraction as other bits.
+static __constant__ float kPackedOne = 1.f;
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r.v)
+      : "l"(b.v), "l"(f2(kPackedOne, kPackedOne).v), "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ void unpack(F2 a, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+
+// one component's running sums c += S * EB (sr.hpp:1151-1369), products and
+// sums rounded separately; a sum starts with its first product (0 + x is x up
+// to the sign of a zero). T is real, or F2 for two components at once; ld(a,
+// b, c) reads tap (a, b, c), Sx, Sy and Sz are the taps' weights.
+template <int D, int O, typename T, typename Ld, typename WX, typename WY, typename WZ>
+__device__ __forceinline__ T interp_sum(Ld&& ld, WX&& Sx, WY&& Sy, WZ&& Sz) {
+  T v;
+#pragma unroll
+  for (int c = 0; c < (D == 3 ? O + 1 : 1); ++c) {
+    T c0;
+#pragma unroll
+    for (int b = 0; b < O + 1; ++b) {
+      T c00;
+#pragma unroll
+      for (int a = 0; a < O + 1; ++a) {
+        const T t = Sx(a) * ld(a, b, c);
+        c00       = a == 0 ? t : c00 + t;
+      }
+      const T t = c00 * Sy(b);
+      c0        = b == 0 ? t : c0 + t;
+    }
+    if constexpr (D == 3) {
+      const T t = c0 * Sz(c);
+      v         = c == 0 ? t : v + t;
+    } else {
+      v = c0;
+    }
+  }
+  return v;
+}
+
 template <int D, int O, typename real, typename V>
 __device__ __forceinline__ void interp_shape(const V& EB, const int* ic,
                                              const real* dc, real* e0, real* b0) {
-  // sr.hpp:1151-1369; running sums c += S * EB, rounded separately
-  int  pmin[3] = { 0, 0, 0 }, dmin[3] = { 0, 0, 0 };
-  real Sp[3][O + 1], Sd[3][O + 1];
+  // first node and weights per axis, [0] primal and [1] dual
+  int  mn[2][3] = { { 0, 0, 0 }, { 0, 0, 0 } };
+  real S[2][3][O + 1];
 #pragma unroll
   for (int a = 0; a < D; ++a) {
-    shape<O, false>(ic[a], dc[a], pmin[a], Sp[a]);
-    shape<O, true>(ic[a], dc[a], dmin[a], Sd[a]);
+    shape<O, false>(ic[a], dc[a], mn[0][a], S[0][a]);
+    shape<O, true>(ic[a], dc[a], mn[1][a], S[1][a]);
+  }
+  real out[6];
+  if constexpr (sizeof(real) == 4) {
+    // Two components per packed operation, those of like staggering along x1
+    // and x2 together: (ex1, bx2), (ex2, bx1) and the odd pair (ex3, bx3). The
+    // order-2 3D interpolation is 468 scalar operations, 195 packed ones.
+#pragma unroll
+    for (int pr = 0; pr < 3; ++pr) {
+      const int ca = pr, cb = pr == 0 ? 4 : (pr == 1 ? 3 : 5);
+      const int xa = stag_of(ca, 0), ya = stag_of(ca, 1), za = stag_of(ca, 2);
+      const int xb = stag_of(cb, 0), yb = stag_of(cb, 1), zb = stag_of(cb, 2);
+      F2 X[O + 1], Y[O + 1], Z[O + 1];
+#pragma unroll
+      for (int k = 0; k < O + 1; ++k) {
+        X[k] = f2(S[xa][0][k], S[xb][0][k]);
+        Y[k] = f2(S[ya][1][k], S[yb][1][k]);
+        if constexpr (D == 3) Z[k] = f2(S[za][2][k], S[zb][2][k]);
+      }
+      const F2 r = interp_sum<D, O, F2>(
+        [&](int a, int b, int c) {
+          return f2(EB.ld(mn[xa][0] + a, mn[ya][1] + b, D == 3 ? mn[za][2] + c : 0, ca),
+                    EB.ld(mn[xb][0] + a, mn[yb][1] + b, D == 3 ? mn[zb][2] + c : 0, cb));
+        },
+        [&](int k) { return X[k]; }, [&](int k) { return Y[k]; }, [&](int k) { return Z[k]; });
+      unpack(r, out[ca], out[cb]);
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      const int x = stag_of(c, 0), y = stag_of(c, 1), z = stag_of(c, 2);
+      out[c] = interp_sum<D, O, real>(
+        [&](int a, int b, int k) {
+          return EB.ld(mn[x][0] + a, mn[y][1] + b, D == 3 ? mn[z][2] + k : 0, c);
+        },
+        [&](int k) { return S[x][0][k]; }, [&](int k) { return S[y][1][k]; },
+        [&](int k) { return S[z][2][k]; });
+    }
   }
 #pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    const int s0 = stag_of(c, 0), s1 = stag_of(c, 1), s2 = stag_of(c, 2);
-    const int m0 = s0 ? dmin[0] : pmin[0];
-    const int m1 = s1 ? dmin[1] : pmin[1];
-    real      v  = 0;
-    if constexpr (D == 2) {
-#pragma unroll
-      for (int b = 0; b < O + 1; b++) {
-        real c0 = 0;
-#pragma unroll
-        for (int a = 0; a < O + 1; a++) {
-          c0 = iacc(s0 ? Sd[0][a] : Sp[0][a], EB.ld(m0 + a, m1 + b, 0, c), c0);
-        }
-        v = iacc(c0, s1 ? Sd[1][b] : Sp[1][b], v);
-      }
-    } else {
-      const int m2 = s2 ? dmin[2] : pmin[2];
-#pragma unroll
-      for (int cc = 0; cc < O + 1; cc++) {
-        real c0 = 0;
-#pragma unroll
-        for (int b = 0; b < O + 1; b++) {
-          real c00 = 0;
-#pragma unroll
-          for (int a = 0; a < O + 1; a++) {
-            c00 = iacc(s0 ? Sd[0][a] : Sp[0][a], EB.ld(m0 + a, m1 + b, m2 + cc, c), c00);
-          }
-          c0 = iacc(c00, s1 ? Sd[1][b] : Sp[1][b], c0);
-        }
-        v = iacc(c0, s2 ? Sd[2][cc] : Sp[2][cc], v);
-      }
-    }
-    if (c < 3) e0[c] = v; else b0[c - 3] = v;
+  for (int c = 0; c < 3; ++c) {
+    e0[c] = out[c];
+    b0[c] = out[c + 3];
   }
 }
 
@@ -479,11 +557,38 @@ __device__ __forceinline__ void move_and_bound(Prtl<real>& q, bool massive, real
 // current deposit of one particle: src/kernels/currents_deposit.hpp:108-761
 // `add(i, j, k, c, v)` accumulates v into J at ghost-inclusive (i, j, k).
 // ---------------------------------------------------------------------------
+// An accumulator that can fix the box's first node derives from BoxAdd: its
+// at(i, j, k) returns one that takes node offsets, so an entry's address is
+// the box's plus a constant.
+struct BoxAdd {};
+template <typename Add>
+struct AtBox {
+  Add& add;
+  int  i0, j0, k0;
+  template <typename real>
+  __device__ __forceinline__ void operator()(int i, int j, int k, int c, real v) const {
+    add(i0 + i, j0 + j, k0 + k, c, v);
+  }
+};
+template <typename Add>
+__device__ __forceinline__ auto at_box(Add& add, int i0, int j0, int k0) {
+  if constexpr (std::is_base_of_v<BoxAdd, Add>) return add.at(i0, j0, k0);
+  else                                          return AtBox<Add>{ add, i0, j0, k0 };
+}
+// Extent of the Esirkepov box (orders 1-3): any (each entry's add is
+// predicated on the particle's own extent), O + 1 nodes per axis (the caller
+// has checked support_unmoved), or all O + 2 nodes per axis added without
+// predicates (entries outside the particle's extent are exact zeros; the
+// accumulator must hold them).
+enum Box { BOX_ANY, BOX_UNMOVED, BOX_FULL };
+// FACTORED: the entries as products of two factors (below) instead of the
+// reference's expressions, equal but for rounding
 // Returns false, touching nothing, when the particle's stencil would reach
 // outside the ghost-inclusive extents `ext` (possible only for moves longer
 // than the ghost layers allow, i.e. a time step beyond the CFL limit);
 // ext == nullptr skips the check (the caller guarantees the window).
-template <int D, int O, typename real, bool UNMOVED = false, typename Add>
+template <int D, int O, typename real, int BOX = BOX_ANY, bool FACTORED = BOX != BOX_ANY,
+          typename Add>
 __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const real* vp,
                                                       real weight, real charge, real inv_dt,
                                                       int ng, const int* ext, Add&& add);
@@ -503,25 +608,25 @@ __device__ __forceinline__ void deposit_velocity(const Prtl<real>& q, real dx, r
   vp[2] *= inv_energy;
 }
 
-template <int D, int O, typename real, typename Add>
+template <int D, int O, typename real, bool FACTORED = false, typename Add>
 __device__ __forceinline__ bool deposit_particle(const Prtl<real>& q, real weight, real charge,
                                                  real inv_dt, real dx, int ng, const int* ext,
                                                  Add&& add) {
   real vp[3];
   deposit_velocity<D, real>(q, dx, vp);
-  return deposit_with_velocity<D, O, real>(q, vp, weight, charge, inv_dt, ng, ext, add);
+  return deposit_with_velocity<D, O, real, BOX_ANY, FACTORED>(q, vp, weight, charge, inv_dt, ng,
+                                                              ext, add);
 }
 
 // the deposit proper, given the particle velocity vp (the GR deposit passes
-// its metric velocity, currents_deposit.hpp:138-159). UNMOVED (orders 1-3):
-// the caller has checked support_unmoved, so every axis' box is O + 1 nodes
-// wide and the stencil's extent is known at compile time; the entries and
-// their values are those of the general form.
-template <int D, int O, typename real, bool UNMOVED, typename Add>
+// its metric velocity, currents_deposit.hpp:138-159)
+template <int D, int O, typename real, int BOX, bool FACTORED, typename Add>
 __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const real* vp,
                                                       real weight, real charge, real inv_dt,
                                                       int ng, const int* ext, Add&& add) {
-  static_assert(!UNMOVED || O >= 1, "the zigzag deposit has no support box");
+  constexpr bool UNMOVED = BOX == BOX_UNMOVED;
+  static_assert(BOX == BOX_ANY || O >= 1, "the zigzag deposit has no support box");
+  static_assert(FACTORED || BOX == BOX_ANY, "the reference's form takes any extent");
   const real ONE = 1, HALF = 0.5, INV_2 = 0.5;
   if constexpr (O == 0) {
     if (ext) {
@@ -606,114 +711,204 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
       }
       if (ext && (imin[a] + ng < 0 || imax[a] + ng >= ext[a])) return false;
     }
-    const real THIRD = K<real>::THIRD;
-    const real Q     = coeff * inv_dt;
-    const int  d1 = UNMOVED ? O : imax[0] - imin[0], d2 = UNMOVED ? O : imax[1] - imin[1];
-    const int  i0 = imin[0] + ng, j0 = imin[1] + ng;
-    // Every entry of the (O+2)-wide stencil is computed and only the add is
-    // predicated on the stencil extent: the loops carry no divergent
-    // branches. Each entry's arithmetic is the reference's expression; the
-    // factors that do not depend on the innermost index are formed once.
-    if constexpr (D == 2) {
-      const real QVx3 = coeff * vp[2];
-      real hd0[N], hs0[N];  // HALF * (fS - iS), HALF * (fS + iS) along x1
+    constexpr real THIRD = K<real>::THIRD;
+    const real     Q     = coeff * inv_dt;
+    if constexpr (!FACTORED) {
+      const int  d1 = imax[0] - imin[0], d2 = imax[1] - imin[1];
+      const int  i0 = imin[0] + ng, j0 = imin[1] + ng;
+      // Every entry of the (O+2)-wide stencil is computed and only the add is
+      // predicated on the stencil extent: the loops carry no divergent
+      // branches. Each entry's arithmetic is the reference's expression; the
+      // factors that do not depend on the innermost index are formed once.
+      if constexpr (D == 2) {
+        const real QVx3 = coeff * vp[2];
+        real hd0[N], hs0[N];  // HALF * (fS - iS), HALF * (fS + iS) along x1
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        hd0[i] = HALF * (fS[0][i] - iS[0][i]);
-        hs0[i] = HALF * (fS[0][i] + iS[0][i]);
-      }
-      // jx1: prefix over i (currents_deposit.hpp:496-518, 547-551)
-#pragma unroll
-      for (int j = 0; j < N; ++j) {
-        const real s1 = fS[1][j] + iS[1][j];
-        real       acc = 0;
-#pragma unroll
-        for (int i = 0; i < N - 1; ++i) {
-          const real W = hd0[i] * s1;
-          acc          = (i == 0) ? (-Q * W) : (acc - Q * W);
-          if (i < d1 && j <= d2) add(i0 + i, j0 + j, 0, 0, acc);
+        for (int i = 0; i < N; ++i) {
+          hd0[i] = HALF * (fS[0][i] - iS[0][i]);
+          hs0[i] = HALF * (fS[0][i] + iS[0][i]);
         }
-      }
-      // jx2: prefix over j
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        real acc = 0;
-#pragma unroll
-        for (int j = 0; j < N - 1; ++j) {
-          const real W = hs0[i] * (fS[1][j] - iS[1][j]);
-          acc          = (j == 0) ? (-Q * W) : (acc - Q * W);
-          if (i <= d1 && j < d2) add(i0 + i, j0 + j, 0, 1, acc);
-        }
-      }
-      // jx3
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        const real ga = HALF * iS[0][i] + fS[0][i];
-        const real gb = HALF * fS[0][i] + iS[0][i];
+        // jx1: prefix over i (currents_deposit.hpp:496-518, 547-551)
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-          const real W = THIRD * (fS[1][j] * ga + iS[1][j] * gb);
-          if (i <= d1 && j <= d2) add(i0 + i, j0 + j, 0, 2, QVx3 * W);
-        }
-      }
-    } else {
-      const int d3 = UNMOVED ? O : imax[2] - imin[2];
-      const int k0 = imin[2] + ng;
-      real      t0[N], t1[N], t2[N];  // THIRD * (fS - iS) per axis
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        t0[i] = THIRD * (fS[0][i] - iS[0][i]);
-        t1[i] = THIRD * (fS[1][i] - iS[1][i]);
-        t2[i] = THIRD * (fS[2][i] - iS[2][i]);
-      }
-      // jx1: prefix over i (currents_deposit.hpp:620-700, 716-724)
-#pragma unroll
-      for (int j = 0; j < N; ++j) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          const real P = (iS[1][j] * iS[2][k] + fS[1][j] * fS[2][k]) +
-                         HALF * (iS[2][k] * fS[1][j] + iS[1][j] * fS[2][k]);
-          const bool ok = (j <= d2) && (k <= d3);
+          const real s1 = fS[1][j] + iS[1][j];
           real       acc = 0;
 #pragma unroll
           for (int i = 0; i < N - 1; ++i) {
-            const real W = t0[i] * P;
+            const real W = hd0[i] * s1;
             acc          = (i == 0) ? (-Q * W) : (acc - Q * W);
-            if (ok && i < d1) add(i0 + i, j0 + j, k0 + k, 0, acc);
+            if (i < d1 && j <= d2) add(i0 + i, j0 + j, 0, 0, acc);
           }
         }
-      }
-      // jx2: prefix over j
+        // jx2: prefix over j
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          const real P = iS[0][i] * iS[2][k] + fS[0][i] * fS[2][k] +
-                         HALF * (iS[2][k] * fS[0][i] + iS[0][i] * fS[2][k]);
-          const bool ok = (i <= d1) && (k <= d3);
-          real       acc = 0;
+        for (int i = 0; i < N; ++i) {
+          real acc = 0;
 #pragma unroll
           for (int j = 0; j < N - 1; ++j) {
-            const real W = t1[j] * P;
+            const real W = hs0[i] * (fS[1][j] - iS[1][j]);
             acc          = (j == 0) ? (-Q * W) : (acc - Q * W);
-            if (ok && j < d2) add(i0 + i, j0 + j, k0 + k, 1, acc);
+            if (i <= d1 && j < d2) add(i0 + i, j0 + j, 0, 1, acc);
+          }
+        }
+        // jx3
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const real ga = HALF * iS[0][i] + fS[0][i];
+          const real gb = HALF * fS[0][i] + iS[0][i];
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            const real W = THIRD * (fS[1][j] * ga + iS[1][j] * gb);
+            if (i <= d1 && j <= d2) add(i0 + i, j0 + j, 0, 2, QVx3 * W);
+          }
+        }
+      } else {
+        const int d3 = imax[2] - imin[2];
+        const int k0 = imin[2] + ng;
+        real      t0[N], t1[N], t2[N];  // THIRD * (fS - iS) per axis
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          t0[i] = THIRD * (fS[0][i] - iS[0][i]);
+          t1[i] = THIRD * (fS[1][i] - iS[1][i]);
+          t2[i] = THIRD * (fS[2][i] - iS[2][i]);
+        }
+        // jx1: prefix over i (currents_deposit.hpp:620-700, 716-724)
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+#pragma unroll
+          for (int k = 0; k < N; ++k) {
+            const real P = (iS[1][j] * iS[2][k] + fS[1][j] * fS[2][k]) +
+                           HALF * (iS[2][k] * fS[1][j] + iS[1][j] * fS[2][k]);
+            const bool ok = (j <= d2) && (k <= d3);
+            real       acc = 0;
+#pragma unroll
+            for (int i = 0; i < N - 1; ++i) {
+              const real W = t0[i] * P;
+              acc          = (i == 0) ? (-Q * W) : (acc - Q * W);
+              if (ok && i < d1) add(i0 + i, j0 + j, k0 + k, 0, acc);
+            }
+          }
+        }
+        // jx2: prefix over j
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+#pragma unroll
+          for (int k = 0; k < N; ++k) {
+            const real P = iS[0][i] * iS[2][k] + fS[0][i] * fS[2][k] +
+                           HALF * (iS[2][k] * fS[0][i] + iS[0][i] * fS[2][k]);
+            const bool ok = (i <= d1) && (k <= d3);
+            real       acc = 0;
+#pragma unroll
+            for (int j = 0; j < N - 1; ++j) {
+              const real W = t1[j] * P;
+              acc          = (j == 0) ? (-Q * W) : (acc - Q * W);
+              if (ok && j < d2) add(i0 + i, j0 + j, k0 + k, 1, acc);
+            }
+          }
+        }
+        // jx3: prefix over k
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+#pragma unroll
+          for (int j = 0; j < N; ++j) {
+            const real P = iS[0][i] * iS[1][j] + fS[0][i] * fS[1][j] +
+                           HALF * (iS[0][i] * fS[1][j] + iS[1][j] * fS[0][i]);
+            const bool ok = (i <= d1) && (j <= d2);
+            real       acc = 0;
+#pragma unroll
+            for (int k = 0; k < N - 1; ++k) {
+              const real W = t2[k] * P;
+              acc          = (k == 0) ? (-Q * W) : (acc - Q * W);
+              if (ok && k < d3) add(i0 + i, j0 + j, k0 + k, 2, acc);
+            }
           }
         }
       }
-      // jx3: prefix over k
+    } else {
+      // The reference's products of initial and final shapes, written in the
+      // mean m = (iS + fS) / 2 and the half difference h = (fS - iS) / 2:
+      //   iS iS' + fS fS' + (iS' fS + iS fS') / 2 = 3 (m m' + h h' / 3),
+      // and the prefix sum along the moving axis taken of 2 h once per axis,
+      // not of every entry's product: an entry is one product of its axis'
+      // prefix and its transverse factor. That is 2 operations per transverse
+      // factor and 1 per entry in place of 8 and 3, with fewer roundings on
+      // the way to each entry (the factors are positive sums: no cancellation).
+      // THIRD keeps the reference's single-precision value.
+      constexpr real ONE_THIRD = (real)(1.0 / 3.0);
+      int lim[3] = { 0, 0, 0 };
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
+      for (int a = 0; a < D; ++a) lim[a] = UNMOVED ? O : imax[a] - imin[a];
+      // nodes an axis' loops visit, and whether node i is inside the extent
+      constexpr int NN = UNMOVED ? O + 1 : N;
+      auto node = [&](int a, int i) { return BOX != BOX_ANY || i <= lim[a]; };
+      auto face = [&](int a, int i) { return BOX != BOX_ANY || i < lim[a]; };
+      auto&& to = at_box(add, imin[0] + ng, imin[1] + ng, D == 3 ? imin[2] + ng : 0);
+      real m[D][NN], h[D][NN];
 #pragma unroll
-        for (int j = 0; j < N; ++j) {
-          const real P = iS[0][i] * iS[1][j] + fS[0][i] * fS[1][j] +
-                         HALF * (iS[0][i] * fS[1][j] + iS[1][j] * fS[0][i]);
-          const bool ok = (i <= d1) && (j <= d2);
-          real       acc = 0;
+      for (int a = 0; a < D; ++a)
 #pragma unroll
-          for (int k = 0; k < N - 1; ++k) {
-            const real W = t2[k] * P;
-            acc          = (k == 0) ? (-Q * W) : (acc - Q * W);
-            if (ok && k < d3) add(i0 + i, j0 + j, k0 + k, 2, acc);
+        for (int i = 0; i < NN; ++i) {
+          m[a][i] = HALF * (fS[a][i] + iS[a][i]);
+          h[a][i] = HALF * (fS[a][i] - iS[a][i]);
+        }
+      // A[i] = c (h[0] + .. + h[i]) along axis a; past the particle's own extent
+      // the sum is zero but for rounding, and BOX_FULL makes it so
+      auto prefix = [&](int a, real c, real* A) {
+        real pre = 0;
+#pragma unroll
+        for (int i = 0; i < NN - 1; ++i) {
+          pre  = i == 0 ? h[a][0] : pre + h[a][i];
+          A[i] = c * pre;
+        }
+        if constexpr (BOX == BOX_FULL) A[NN - 2] = NN - 2 < lim[a] ? A[NN - 2] : (real)0;
+      };
+      if constexpr (D == 2) {
+        real A[NN - 1];
+        // jx1: prefix over i (currents_deposit.hpp:496-518, 547-551):
+        // -Q (fS - iS) / 2 (fS' + iS') = (-2 Q) h m'
+        prefix(0, (real)-2 * Q, A);
+#pragma unroll
+        for (int i = 0; i < NN - 1; ++i)
+#pragma unroll
+          for (int j = 0; j < NN; ++j)
+            if (face(0, i) && node(1, j)) to(i, j, 0, 0, A[i] * m[1][j]);
+        // jx2: prefix over j
+        prefix(1, (real)-2 * Q, A);
+#pragma unroll
+        for (int j = 0; j < NN - 1; ++j)
+#pragma unroll
+          for (int i = 0; i < NN; ++i)
+            if (node(0, i) && face(1, j)) to(i, j, 0, 1, A[j] * m[0][i]);
+        // jx3: Q v3 THIRD (fS1 (iS0 / 2 + fS0) + iS1 (fS0 / 2 + iS0))
+        const real q3 = (coeff * vp[2]) * ((real)3 * THIRD);
+#pragma unroll
+        for (int i = 0; i < NN; ++i) {
+          const real qm = q3 * m[0][i], qh = (q3 * ONE_THIRD) * h[0][i];
+#pragma unroll
+          for (int j = 0; j < NN; ++j)
+            if (node(0, i) && node(1, j)) to(i, j, 0, 2, fma(qh, h[1][j], qm * m[1][j]));
+        }
+      } else {
+        const real c6 = (real)-6 * THIRD * Q;
+        // component a: prefix along axis a, transverse factor of the axes b < c
+        // (currents_deposit.hpp:620-754)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+          real      A[NN - 1];
+          prefix(a, c6, A);
+#pragma unroll
+          for (int k = 0; k < NN; ++k) {
+            const real hk = ONE_THIRD * h[c][k], mk = m[c][k];
+#pragma unroll
+            for (int j = 0; j < NN; ++j) {
+              const real P  = fma(hk, h[b][j], mk * m[b][j]);
+              const bool ok = node(b, j) && node(c, k);
+#pragma unroll
+              for (int i = 0; i < NN - 1; ++i)
+                if (ok && face(a, i))
+                  to(a == 0 ? i : j, a == 1 ? i : (a == 0 ? j : k), a == 2 ? i : k, a, A[i] * P);
+            }
           }
         }
       }

@@ -9,9 +9,10 @@
 //      particles' weights, or a strided copy loop for a window that wraps
 //      across a periodic edge;
 //   2. pushes every particle of the tile (all species) gathering E/B from
-//      shared memory and depositing its current into a shared-memory J window
-//      (tile + deposit halo + margin); in FP32 a particle whose shape
-//      support moved is deposited after the pushes, from a record (DepStage),
+//      shared memory, and deposits its current into a shared-memory J window
+//      (tile + deposit halo + margin); at orders 1-3 from records, after the
+//      pushes (DepStage: every particle in 3D, in 2D those whose shape support
+//      moved),
 //   3. adds the J window to global J once, wrapping periodic images onto
 //      their active cells (the fold SynchronizeFields performs in the
 //      reference, src/framework/domain/metadomain_comm.cpp:408-562).
@@ -38,8 +39,8 @@
 // overflow list and pushed afterwards by the per-particle kernel (global
 // gathers, global atomics, the reference's coordinates). Results therefore
 // never depend on the sort interval, and the hot kernel holds only the
-// shared-memory path. Arithmetic per particle is the same code as the
-// untiled kernel.
+// shared-memory path. The push is the same code as the untiled kernel's, the
+// deposit its factored form (pic_common.cuh), equal but for rounding.
 #pragma once
 
 #include <type_traits>
@@ -121,30 +122,29 @@ struct TileShape {
   // (4 CTAs), 0.350 ms at 48 (5 CTAs, no spill) and 0.366 ms at 40 (6 CTAs,
   // spilling); 512 threads x 2 gave 0.408 ms
   static constexpr int X = 16, Y = 8, Z = 1, NT = 256,
-                       MINB = sizeof(real) == 4 ? (O == 3 ? 4 : 5) : 1;  // order 3 spills at 5
+                       MINB = sizeof(real) == 4 ? (O == 3 ? 4 : 5) : 1,  // order 3 spills at 5
+                       CHUNK = 2048;
 };
-// 3D FP32 at order 3: 8^3 cells, so that two copies of the J window fit
-// (measured on the 96^3 sweep plasma, 2 x 32 ppc: 28.1 ms per step against
-// 34.7 ms with one copy and 16 x 8 x 4 tiles). At order 2 the copies did not
-// pay (50.5 against 48.1 ms on the 256^3 turbulence plasma, 2 x 8 ppc; with
-// the deposit records and the even-odd rows 34.5 against 28.8 ms): its warps
-// span several cells, so fewer lanes share a word.
-// Threads per CTA: one CTA per SM (the shared memory), so the thread count
-// sets the warps that hide the kernel's latencies, and the register file
-// sets what each may use. Push+deposit of the 256^3 turbulence plasma
-// (order 2) took 44.96 ms at 512 threads (128 registers), 40.26 at 640 (96),
-// 38.38 at 768 (80), 38.19 at 896 (72) and 36.31 at 1024 (64, no spill); the
-// 96^3 sweep plasma (order 3) 27.00, 25.55, 25.62, 26.30 and 26.86 ms (at
-// 1024 its registers spill)
+// 3D FP32. One CTA per SM (the shared memory), so the thread count sets the
+// warps that hide the kernel's latencies, and the register file what each may
+// use. Steps of the 256^3 turbulence plasma (order 2, 2 x 8 ppc) took 26.8 ms
+// with 768 threads (80 registers) and 26.7 with 1024 (64); steps of the 96^3
+// sweep plasma (order 3, 2 x 32 ppc) 12.5, 12.0 and 11.9 ms with 640, 768 and
+// 1024. CHUNK: particles pushed between deposits. More of them fill the
+// records' classes more evenly and wait at fewer barriers: 5120, 10240 and
+// 20480 (more than a tile of the turbulence plasma holds) gave 28.9, 26.7 and
+// 25.6 ms, 20480 and 36864 (a tile of the sweep plasma) 11.9 and 11.6 ms.
 template <int O>
 struct TileShape<3, float, O> {
-  static constexpr int X = (O == 3 ? 8 : 16), Y = 8, Z = 8, NT = (O == 3 ? 640 : 1024), MINB = 1;
+  static constexpr int X = (O == 3 ? 8 : 16), Y = 8, Z = 8, NT = 1024, MINB = 1,
+                       CHUNK = (O == 3 ? 36 : 20) * 1024;
 };
-// FP64 (8 x 8 x 4 cells): 256, 384, 512 and 768 threads ran the FP64 twin of
-// the sweep plasma (order 3) at 150, 151, 145 and 137 M particle-steps/s
+// FP64 (8 x 8 x 4 cells) is bound by the FP64 pipe (two lanes per SM and
+// clock): 384 and 512 threads, chunks of 4608 and 5120 particles all gave
+// 10.1 to 10.2 ms per step of the 64^3 turbulence box
 template <int O>
 struct TileShape<3, double, O> {
-  static constexpr int X = 8, Y = 8, Z = 4, NT = 384, MINB = 1;
+  static constexpr int X = 8, Y = 8, Z = 4, NT = 384, MINB = 1, CHUNK = 4608;
 };
 
 // window halos (cells below / above the tile) of the interpolation and the
@@ -167,26 +167,35 @@ struct TiledSpecies {
   unsigned*      ovf_count;
 };
 
-// Deposit records (FP32: 3D orders 1-3, 2D orders 1-2; 2D records carry the
-// out-of-plane velocity in place of the third offsets). Most particles end a
-// step with both shape supports starting at the same node on every axis
-// (support_unmoved): their Esirkepov box is (O + 1) wide on each axis, a
-// stencil the compiler unrolls to its exact extent (54 of the 144 entries at
-// order 2). A warp deposits those at once. The others, whose box is O + 2
-// wide on some axis, are appended as 32-byte records to a buffer in global
-// memory (L2-resident: a few hundred KB per CTA, written and read back by
-// the same CTA) and deposited after the tile's pushes by full warps. So no
-// warp runs the wide stencil for one lane, and J is unchanged to the bit:
-// the window's integer sums do not depend on the order of the additions.
-// A CTA claims one of nslots buffers (nslots >= the CTAs that can be
-// resident at once); without one, or past cap records, it deposits at once.
+// Deposit records (orders 1-3). A particle's push appends a 32-byte record
+// (48 in FP64: cell offsets from the tile, the offsets before and after the
+// move, q w, in 2D the out-of-plane velocity) to a buffer in global memory
+// (L2-resident, written and read back by the same CTA), and the CTA deposits
+// the records once it has pushed a chunk of its particles.
+//   - The records are queued by bank class, the shared-memory bank (of 32) of
+//     the first J-window word of the particle's Esirkepov box. Row r of a
+//     buffer holds the r-th record of each class, and a warp takes a row: its
+//     32 lanes add to entries at the same offsets from 32 first words in 32
+//     different banks, so every atomic of the warp is one wavefront. Deposited
+//     in cell order, lanes of one cell serialise on its words (3.6 wavefronts
+//     per atomic on the turbulence plasma, the shared pipe at 65 % of its
+//     peak).
+//   - Most particles end a step with both shape supports starting at the same
+//     node on every axis (support_unmoved): their box is (O + 1) wide on each
+//     axis, a stencil the compiler unrolls to its exact extent (54 of the 144
+//     entries at order 2 in 3D). The others, whose box is O + 2 wide on some
+//     axis, have rows of their own, so no warp runs the wide stencil for one
+//     lane.
+// J does not depend on the records to the bit: the window's integer sums are
+// independent of the order of the additions. A full class hands its records
+// to the next one, which costs a bank conflict; the rows of a region hold a
+// whole chunk, so a record always finds a place. A CTA claims one of nslots
+// buffers; there are as many as CTAs that can be resident at once.
 struct DepStage {
-  uint4*    rec    = nullptr;  // nslots * cap records of two uint4
+  uint4*    rec    = nullptr;  // nslots buffers of two regions (unmoved, moved)
   unsigned* claim  = nullptr;  // nslots words: 0 free, 1 held
-  int       nslots = 0, cap = 0;
+  int       nslots = 0;
 };
-// records per 3D buffer (256 KB); twice that at order 3, a quarter in 2D
-constexpr int kStageCap = 8192;
 
 // drops the 128-byte line at p (128-byte aligned) from L2 without writing it
 // back; its contents are undefined until written again
@@ -214,15 +223,11 @@ struct TiledArgs {
   // FP32: the exact 64-bit accumulator the tile sums are flushed into (null:
   // float atomics into J)
   FixedJ             fj;
-  // 3D FP32: where a tile's moved-support particles wait for their deposit
+  // where a tile's pushed particles wait for their deposit
   DepStage           st;
   // warps taken lane_stride at a time read their particles interleaved
-  // (1, 2 or 4; a divisor of the CTA's warps). A warp of a cell-sorted tile
-  // then spans 32 lane_stride / ppc cells; about four measured best: on
-  // the 256^3 turbulence plasma (8 ppc per species) strides 1, 2 and 4 took
-  // 28.9, 29.6 and 30.4 ms of push+deposit, on the 96^3 sweep plasma (32)
-  // 24.1, 21.2 and 20.4 ms, on the 512^2 pair plasma (16) 0.333, 0.323 and
-  // 0.330 ms
+  // (1, 2 or 4; a divisor of the CTA's warps): a warp of a cell-sorted tile
+  // then spans 32 lane_stride / ppc cells (the rule is with the caller)
   int                lane_stride = 1;
 };
 
@@ -239,30 +244,27 @@ struct TiledGeom {
   static constexpr int WJ1 = TY + H::J_LO + H::J_HI;
   static constexpr int WJ2 = D == 3 ? TZ + H::J_LO + H::J_HI : 1;
   static constexpr int NJ  = WJ0 * WJ1 * WJ2;
-  // J window: FixedAcc<real>::WORDS planes of 3 * NJ 32-bit words, in COPIES
-  // copies (3D FP32 at order 3: two, one per lane parity) COPY words apart.
-  // Two copies in 2D FP32 did not pay: the 512^2 pair plasma's push+deposit
-  // took 0.325 ms against 0.322 ms with one
+  // J window: FixedAcc<real>::WORDS planes of 3 * NJ 32-bit words
   static constexpr int    WORDS      = FixedAcc<real>::WORDS;
   static constexpr int    PLANE      = 3 * NJ;
-  static constexpr int    COPIES     = (D == 3 && sizeof(real) == 4 && O == 3) ? 2 : 1;
-  // moved-support particles deposited from records (DepStage), orders 1-3.
-  // At order 3 the buffers hold twice the records: the sweep plasma
-  // (theta = 1, 8^3-cell tiles of 2 x 32 ppc) moves 40 % of its supports;
-  // with 8192 records per buffer its push+deposit on 96^3 went from 25.0 to
-  // 27.5 ms, with 16384 (and the lane stride) from 20.5 to 19.6 ms
-  // 2D at order 3 would spill at its four CTAs per SM, so it deposits at once
-  static constexpr bool   STAGE      = sizeof(real) == 4 && O >= 1 && (D == 3 || O <= 2);
-  // the copies start 16 banks apart: one word in both copies falls in
-  // two different banks
-  static constexpr int    COPY       = WORDS * PLANE + ((16 - (WORDS * PLANE) % 32) + 32) % 32;
-  static constexpr size_t jw_bytes   = 4 * (size_t)(COPIES == 1 ? WORDS * PLANE : COPIES * COPY);
+  static constexpr size_t jw_bytes   = 4 * (size_t)(WORDS * PLANE);
+  // Deposit records: all particles' (REC_ALL), or those of particles whose
+  // support moved, the others depositing at once
+  static constexpr bool   REC        = O >= 1;
+  static constexpr bool   REC_ALL    = D == 3;
+  static constexpr int    RECW       = sizeof(real) == 4 ? 2 : 3;  // 16-byte words per record
+  static constexpr int    CHUNK      = TS::CHUNK;                  // particles between deposits
+  static constexpr int    ROWS       = CHUNK / 32;                 // rows per region
+  static constexpr size_t region     = (size_t)CHUNK * RECW;       // 16-byte words
+  static constexpr size_t moved      = REC_ALL ? region : 0;       // start of the moved region
+  static constexpr size_t slot_words = moved + region;
+  static_assert(CHUNK % 32 == 0 && CHUNK >= NT, "a chunk holds one particle per thread at least");
   // E window rows: a TMA box row is a multiple of 16 bytes and starts on a
   // 16-byte boundary, so the row is widened to WEX elements and the window
   // sits R = (x start mod A) elements into it (A elements per 16 bytes)
   static constexpr int    A          = 16 / (int)sizeof(real);
   static constexpr int    WEX_TMA    = ((WE0 + A - 1 + A - 1) / A) * A;
-  static constexpr size_t kSmemMax   = 232448 - 128;  // per-CTA limit less the static words
+  static constexpr size_t kSmemMax   = 232448 - 512;  // per-CTA limit less the static words
   static constexpr bool fits(int wx, int wy) {
     return ((sizeof(real) * 6 * (size_t)wx * wy * WE2 + 127) / 128) * 128 + jw_bytes <= kSmemMax;
   }
@@ -296,13 +298,42 @@ struct TiledGeom {
   static constexpr size_t smem_bytes = ((eb_bytes + 127) / 128) * 128 + jw_bytes;
 };
 
+// J-window accumulators: base is the word of ghost-inclusive node (0, 0, 0)
+template <typename G, typename FA>
+struct JWinFixed : BoxAdd {
+  unsigned* w;
+  int       base;
+  __device__ __forceinline__ JWinFixed(unsigned* w_, int b) : w(w_), base(b) {}
+  __device__ __forceinline__ JWinFixed at(int i, int j, int k) const {
+    return { w, base + i + j * G::WJ0 + k * (G::WJ0 * G::WJ1) };
+  }
+  template <typename real>
+  __device__ __forceinline__ void operator()(int i, int j, int k, int c, real v) const {
+    FA::add(w + base + (i + j * G::WJ0 + k * (G::WJ0 * G::WJ1) + c * G::NJ), G::PLANE, v);
+  }
+};
+template <typename G, typename real>
+struct JWinReal : BoxAdd {
+  real* w;
+  int   base;
+  __device__ __forceinline__ JWinReal(real* w_, int b) : w(w_), base(b) {}
+  __device__ __forceinline__ JWinReal at(int i, int j, int k) const {
+    return { w, base + i + j * G::WJ0 + k * (G::WJ0 * G::WJ1) };
+  }
+  __device__ __forceinline__ void operator()(int i, int j, int k, int c, real v) const {
+    atomicAdd(w + base + (i + j * G::WJ0 + k * (G::WJ0 * G::WJ1) + c * G::NJ), v);
+  }
+};
+
 // wraps a ghost-free coordinate of a periodic axis into [0, n)
 __device__ __forceinline__ int wrap_periodic(int x, int n) {
   x %= n;
   return x < 0 ? x + n : x;
 }
 
-template <int D, int O, typename real>
+// REC: deposits go through records (DepStage); without, every particle
+// deposits as it is pushed (order 0, or no buffers)
+template <int D, int O, typename real, bool REC>
 __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, O>::MINB)
     k_push_deposit_tiled(const __grid_constant__ TiledArgs<real> a) {
   using G               = TiledGeom<D, O, real>;
@@ -316,8 +347,8 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
   real*          Jr  = reinterpret_cast<real*>(Jw);  // real_t accumulation of dense tiles
   __shared__ unsigned int s_qmax;  // bit pattern of the tile's largest |q w| max(1/dt, 1)
   __shared__ __align__(8) unsigned long long s_bar;  // completion of the E-window load
-  __shared__ int      s_slot;  // the claimed record buffer, -1 for none
-  __shared__ unsigned s_nrec;  // records appended so far
+  __shared__ int      s_slot;         // the claimed record buffer, -1 for none
+  __shared__ unsigned s_cnt[2][32];   // records per class, unmoved and moved supports
 
   const int t  = blockIdx.x + a.tile0;
   const int tx = t % a.ntiles[0];
@@ -376,24 +407,31 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
           inside ? a.EB.ld(gc[0] + ng, gc[1] + ng, D == 3 ? gc[2] + ng : 0, c) : (real)0;
     }
   }
-  for (int idx = threadIdx.x; idx < (G::COPIES == 1 ? G::WORDS * G::PLANE : G::COPIES * G::COPY);
-       idx += NT)
+  for (int idx = threadIdx.x; idx < G::WORDS * G::PLANE; idx += NT)
     Jw[idx] = 0u;
   // largest contribution bound of the tile, |q w| max(1/dt, 1), and its
   // particle count (an upper bound on the additions any cell receives)
+  if constexpr (REC) {
+    if (threadIdx.x < 64) (&s_cnt[0][0])[threadIdx.x] = 0u;
+  }
   if (threadIdx.x == 0) {
     s_qmax = 0u;
-    s_nrec = 0u;
     s_slot = -1;
-    if (G::STAGE && a.st.rec) {
-      // one attempt per buffer, starting where this CTA's predecessors by
-      // index left theirs: no wait
-      for (int k = 0; k < a.st.nslots; ++k) {
-        const int sl = (int)((blockIdx.x + (unsigned)k) % (unsigned)a.st.nslots);
+    if constexpr (REC) {
+      // nslots is a multiple of the SMs: the search starts with this SM's own
+      // buffers, one of which its last CTA has just given back. The limit
+      // bounds the search all the same.
+      unsigned sm, nsm;
+      asm("mov.u32 %0, %%smid;" : "=r"(sm));
+      asm("mov.u32 %0, %%nsmid;" : "=r"(nsm));
+      const unsigned n = (unsigned)a.st.nslots, per = max(1u, n / max(1u, nsm));
+      unsigned       sl = (sm * per) % n;
+      for (unsigned k = 0; k < 64u * n; ++k) {
         if (atomicCAS(a.st.claim + sl, 0u, 1u) == 0u) {
-          s_slot = sl;
+          s_slot = (int)sl;
           break;
         }
+        if (++sl == n) sl = 0;
       }
     }
   }
@@ -427,14 +465,15 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
   scale   = (real)ldexp(1.0, b - ex);
   unscale = (real)ldexp(1.0, ex - b);
 
-  if (tma) {
+  {
     // every thread waits for the window; a lost wait (the limit ran out on
     // any thread) abandons the tile on all of them and is counted
-    const bool done = mbar_wait_bounded(bar, 0u);
+    bool done = !tma || mbar_wait_bounded(bar, 0u);
+    if constexpr (REC) done = done && s_slot >= 0;
     if (__syncthreads_or(!done)) {
       if (threadIdx.x == 0) {
         atomicAdd(a.err + ERR_WAIT_TIMEOUT, 1ull);
-        if (s_slot >= 0) atomicExch(a.st.claim + s_slot, 0u);
+        if (REC && s_slot >= 0) atomicExch(a.st.claim + s_slot, 0u);
       }
       return;
     }
@@ -443,210 +482,248 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
   const int joff[3] = { ng + T0[0] - H::J_LO, ng + T0[1] - H::J_LO,
                         D == 3 ? ng + T0[2] - H::J_LO : 0 };
   const int jb      = -joff[0] - joff[1] * G::WJ0 - joff[2] * (G::WJ0 * G::WJ1);
-  const int slot    = s_slot;
-  // The thread's particle within each NT-particle chunk. With lane_stride
+  // The thread's particle within each NT-particle group. With lane_stride
   // ls, ls consecutive warps share 32 ls consecutive particles, lane l of the
   // group's k-th warp taking particle ls l + k: each warp spans ls times as
   // many cells, so fewer of its lanes add to one J word, and the group
   // still reads whole lines.
   const int ls      = a.lane_stride;
+  const int lane    = (int)(threadIdx.x & 31);
   const int wid     = (int)(threadIdx.x >> 5);
-  const int local   = (wid / ls) * (32 * ls) + ls * (int)(threadIdx.x & 31) + wid % ls;
-  uint4*    recs    = slot >= 0 ? a.st.rec + (size_t)slot * a.st.cap * 2 : nullptr;
+  const int local   = (wid / ls) * (32 * ls) + ls * lane + wid % ls;
+  uint4*    recs    = REC ? a.st.rec + (size_t)s_slot * G::slot_words : nullptr;
   // cell of a record relative to the tile: 8 bits per axis, offset by 64
   static_assert(G::TX + kDriftMargin + 2 < 64 && G::TY + kDriftMargin + 2 < 64 &&
                     G::TZ + kDriftMargin + 2 < 64,
                 "record cells are 8-bit offsets from the tile origin");
+  // the two accumulations, chosen once per deposit: a test at every entry
+  // cost the order-2 kernel a sixth of its instructions
+  const JWinFixed<G, FA>   add_fixed{ Jw, jb };
+  const JWinReal<G, real> add_real{ Jr, jb };
 
-  // 2. particles of the tile, species by species
-  for (int s = 0; s < a.nsp; ++s) {
-    const TiledSpecies<real>& S = a.s[s];
-    real*          ux[3]  = { (real*)S.sp.ux1, (real*)S.sp.ux2, (real*)S.sp.ux3 };
-    const real*    w      = (const real*)S.sp.w;
-    int32_t*       ia[3]  = { S.sp.i1, S.sp.i2, S.sp.i3 };
-    int32_t*       ipa[3] = { S.sp.i1p, S.sp.i2p, S.sp.i3p };
-    float*         da[3]  = { S.sp.dx1, S.sp.dx2, S.sp.dx3 };
-    float*         dpa[3] = { S.sp.dx1p, S.sp.dx2p, S.sp.dx3p };
-    const int64_t  lo = S.tile_start[t], hi = S.tile_start[t + 1];
-    for (int64_t p = lo + local; p < hi; p += NT) {
-      Prtl<real> q;
-      q.tag = S.sp.tag[p];
-      if (q.tag != PIC_TAG_ALIVE) {
-        if (q.tag != PIC_TAG_DEAD) atomicAdd(a.err + ERR_BAD_TAG, 1ull);
-        continue;
-      }
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        q.i[d]  = ia[d][p];
-        q.dx[d] = da[d][p];
-      }
-      if (!cells_in_grid<D>(q.i, a.pc.n)) {
-        atomicAdd(a.err + ERR_OUT_OF_GRID, 1ull);
-        continue;
-      }
-      bool near = true, edge = false;
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        const int T = d == 0 ? G::TX : (d == 1 ? G::TY : G::TZ);
-        near = near && (q.i[d] >= T0[d] - M) && (q.i[d] < T0[d] + T + M);
-        // a stencil that can reach the ghost layers of a non-periodic axis is
-        // deposited at the reference's coordinates: there the reference keeps
-        // the raw ghost currents, unfolded along the periodic axes
-        edge = edge || (!a.periodic[d] &&
-                        (q.i[d] < H::J_LO - M + 1 || q.i[d] >= a.pc.n[d] - (H::J_HI - M) - 1));
-      }
-      {
-        // particles that drifted past the margin, or whose stencil can reach
-        // the ghost layers of a non-periodic axis, are left to the
-        // per-particle kernel (global gathers, reference coordinates)
-        const bool     defer = !near || edge;
-        const unsigned ball  = __ballot_sync(__activemask(), defer);
-        if (defer) {
-          const int      lane   = threadIdx.x & 31;
-          const int      leader = __ffs(ball) - 1;
-          unsigned       base   = 0;
-          if (lane == leader) base = atomicAdd(S.ovf_count, (unsigned)__popc(ball));
-          base = __shfl_sync(ball, base, leader);
-          S.ovf[base + __popc(ball & ((1u << lane) - 1u))] = (int32_t)p;
-          continue;
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) q.u[d] = ux[d][p];
-      real e0[3], b0[3];
-      int  ic[3] = { q.i[0] + ng, q.i[1] + ng, D == 3 ? q.i[2] + ng : 0 };
-      real dc[3] = { (real)q.dx[0], (real)q.dx[1], D == 3 ? (real)q.dx[2] : (real)0 };
-      if constexpr (O == 0) interp_zigzag<D, real>(ebv, ic, dc, e0, b0);
-      else                  interp_shape<D, O, real>(ebv, ic, dc, e0, b0);
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        e0[d] = e0[d] * a.dx;
-        b0[d] = b0[d] * a.dx;
-      }
-      if (S.vay) vay<real>(S.ndth, q.u, e0, b0);
-      else       boris<real>(S.ndth, q.u, e0, b0);
-      move_and_bound<D, real>(q, true, a.dt, a.dx, a.pc);
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        ia[d][p] = q.i[d];
-        da[d][p] = q.dx[d];
-      }
-#pragma unroll
-      for (int d = 0; d < 3; ++d) ux[d][p] = q.u[d];
-      if (q.tag != PIC_TAG_ALIVE) S.sp.tag[p] = q.tag;
-      if (a.write_prev) {
+  // 2. particles of the tile, species by species; with records in chunks,
+  //    each pushed by the whole CTA and then deposited
+  int     s  = 0;
+  int64_t p0 = a.s[0].tile_start[t];  // first particle of the CTA's next group
+  for (;;) {
+    int pend = 0;  // particles since the last deposit, rounded up to groups
+    while (s < a.nsp) {
+      const TiledSpecies<real>& S = a.s[s];
+      real*          ux[3]  = { (real*)S.sp.ux1, (real*)S.sp.ux2, (real*)S.sp.ux3 };
+      const real*    w      = (const real*)S.sp.w;
+      int32_t*       ia[3]  = { S.sp.i1, S.sp.i2, S.sp.i3 };
+      int32_t*       ipa[3] = { S.sp.i1p, S.sp.i2p, S.sp.i3p };
+      float*         da[3]  = { S.sp.dx1, S.sp.dx2, S.sp.dx3 };
+      float*         dpa[3] = { S.sp.dx1p, S.sp.dx2p, S.sp.dx3p };
+      const int64_t  hi = S.tile_start[t + 1];
+      for (; p0 < hi && (!REC || pend + NT <= G::CHUNK); p0 += NT, pend += NT) {
+        const int64_t p = p0 + local;
+        if (p >= hi) continue;
+        // the whole state is loaded before the first test of it: one latency
+        Prtl<real> q;
+        q.tag = S.sp.tag[p];
 #pragma unroll
         for (int d = 0; d < D; ++d) {
-          ipa[d][p] = q.ip[d];
-          dpa[d][p] = q.dxp[d];
+          q.i[d]  = ia[d][p];
+          q.dx[d] = da[d][p];
         }
-      }
-      if (q.tag == PIC_TAG_DEAD || S.charge == (real)0) continue;
-      // deposit at the coordinates before the periodic wrap (a shift of both
-      // i and i_prev by n leaves every contribution unchanged up to the image
-      // cell, which the flush folds back)
 #pragma unroll
-      for (int d = 0; d < D; ++d) {
-        q.i[d] -= q.wrap[d];
-        q.ip[d] -= q.wrap[d];
-      }
-      // in fixed point the weight carries the power-of-two scale, so every
-      // contribution arrives scaled exactly (w 2^s rounds like w)
-      const real wp = fixed ? w[p] * scale : w[p];
-      // Shared-memory atomics serialise the lanes of a warp that hit one
-      // word, and cell-sorted lanes share their boxes: odd and even lanes
-      // add to separate copies, which halves those collisions. The flush
-      // sums the copies' integer totals, so J is unchanged to the bit.
-      unsigned* Jc  = Jw + (G::COPIES == 2 ? (int)(threadIdx.x & 1) * G::COPY : 0);
-      auto      add = [&](int i, int j, int k, int c, real v) {
-        const int e = jb + i + j * G::WJ0 + k * (G::WJ0 * G::WJ1) + c * G::NJ;
-        if (fixed) FA::add(Jc + e, G::PLANE, v);
-        else       atomicAdd(Jr + e, v);
-      };
-      if constexpr (G::STAGE) {
-        if (recs) {
+        for (int d = 0; d < 3; ++d) q.u[d] = ux[d][p];
+        const real wq = w[p];
+        if (q.tag != PIC_TAG_ALIVE) {
+          if (q.tag != PIC_TAG_DEAD) atomicAdd(a.err + ERR_BAD_TAG, 1ull);
+          continue;
+        }
+        if (!cells_in_grid<D>(q.i, a.pc.n)) {
+          atomicAdd(a.err + ERR_OUT_OF_GRID, 1ull);
+          continue;
+        }
+        bool near = true, edge = false;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          const int T = d == 0 ? G::TX : (d == 1 ? G::TY : G::TZ);
+          near = near && (q.i[d] >= T0[d] - M) && (q.i[d] < T0[d] + T + M);
+          // a stencil that can reach the ghost layers of a non-periodic axis is
+          // deposited at the reference's coordinates: there the reference keeps
+          // the raw ghost currents, unfolded along the periodic axes
+          edge = edge || (!a.periodic[d] &&
+                          (q.i[d] < H::J_LO - M + 1 || q.i[d] >= a.pc.n[d] - (H::J_HI - M) - 1));
+        }
+        {
+          // particles that drifted past the margin, or whose stencil can reach
+          // the ghost layers of a non-periodic axis, are left to the
+          // per-particle kernel (global gathers, reference coordinates)
+          const bool     defer = !near || edge;
+          const unsigned ball  = __ballot_sync(__activemask(), defer);
+          if (defer) {
+            const int leader = __ffs(ball) - 1;
+            unsigned  base   = 0;
+            if (lane == leader) base = atomicAdd(S.ovf_count, (unsigned)__popc(ball));
+            base = __shfl_sync(ball, base, leader);
+            S.ovf[base + __popc(ball & ((1u << lane) - 1u))] = (int32_t)p;
+            continue;
+          }
+        }
+        real e0[3], b0[3];
+        int  ic[3] = { q.i[0] + ng, q.i[1] + ng, D == 3 ? q.i[2] + ng : 0 };
+        real dc[3] = { (real)q.dx[0], (real)q.dx[1], D == 3 ? (real)q.dx[2] : (real)0 };
+        if constexpr (O == 0) interp_zigzag<D, real>(ebv, ic, dc, e0, b0);
+        else                  interp_shape<D, O, real>(ebv, ic, dc, e0, b0);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          e0[d] = e0[d] * a.dx;
+          b0[d] = b0[d] * a.dx;
+        }
+        if (S.vay) vay<real>(S.ndth, q.u, e0, b0);
+        else       boris<real>(S.ndth, q.u, e0, b0);
+        move_and_bound<D, real>(q, true, a.dt, a.dx, a.pc);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          ia[d][p] = q.i[d];
+          da[d][p] = q.dx[d];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) ux[d][p] = q.u[d];
+        if (q.tag != PIC_TAG_ALIVE) S.sp.tag[p] = q.tag;
+        if (a.write_prev) {
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            ipa[d][p] = q.ip[d];
+            dpa[d][p] = q.dxp[d];
+          }
+        }
+        if (q.tag == PIC_TAG_DEAD || S.charge == (real)0) continue;
+        // deposit at the coordinates before the periodic wrap (a shift of both
+        // i and i_prev by n leaves every contribution unchanged up to the image
+        // cell, which the flush folds back)
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          q.i[d] -= q.wrap[d];
+          q.ip[d] -= q.wrap[d];
+        }
+        // in fixed point the weight carries the power-of-two scale, so every
+        // contribution arrives scaled exactly (w 2^s rounds like w)
+        const real wp = fixed ? wq * scale : wq;
+        if constexpr (REC) {
           // the 2D deposit reads the out-of-plane velocity, the 3D one none
           real vp[3] = { 0, 0, 0 };
           if constexpr (D == 2) deposit_velocity<D, real>(q, a.dx, vp);
-          if (support_unmoved<D, O, real>(q)) {
-            deposit_with_velocity<D, O, real, true>(q, vp, wp, S.charge, a.inv_dt, ng, nullptr,
-                                                    add);
+          const bool unmoved = support_unmoved<D, O, real>(q);
+          if (!G::REC_ALL && unmoved) {
+            if (fixed)
+              deposit_with_velocity<D, O, real, BOX_UNMOVED>(q, vp, wp, S.charge, a.inv_dt, ng, nullptr,
+                                                      add_fixed);
+            else
+              deposit_with_velocity<D, O, real, BOX_UNMOVED>(q, vp, wp, S.charge, a.inv_dt, ng, nullptr,
+                                                      add_real);
             continue;
           }
-          // a record needs the move to stay within one cell per axis
-          bool one = true;
+          // first node of the box, as a J-window word (the move stays within
+          // one cell per axis: move_and_bound steps the cell by one at most)
+          int      word  = jb;
+          unsigned cells = 0;
 #pragma unroll
-          for (int d = 0; d < D; ++d) one = one && q.ip[d] - q.i[d] >= -1 && q.ip[d] - q.i[d] <= 1;
-          const unsigned ball = __ballot_sync(__activemask(), one);
-          if (one) {
-            const int lane   = threadIdx.x & 31;
-            const int leader = __ffs(ball) - 1;
-            unsigned  base   = 0;
-            if (lane == leader) base = atomicAdd(&s_nrec, (unsigned)__popc(ball));
-            base             = __shfl_sync(ball, base, leader);
-            const unsigned r = base + __popc(ball & ((1u << lane) - 1u));
-            if (r < (unsigned)a.st.cap) {
-              unsigned cells = 0;
-#pragma unroll
-              for (int d = 0; d < D; ++d)
-                cells |= ((unsigned)(q.i[d] - T0[d] + 64) << (8 * d)) |
-                         ((unsigned)(q.ip[d] - q.i[d] + 1) << (24 + 2 * d));
-              const float coeff = (float)(wp * S.charge);
-              // 3D: the offsets x3 in the third words; 2D: the out-of-plane
-              // velocity in their place
-              const float w3 = D == 3 ? q.dx[2] : (float)vp[2], p3 = D == 3 ? q.dxp[2] : 0.f;
-              __stcg(recs + 2 * r, make_uint4(cells, __float_as_uint(q.dx[0]),
-                                              __float_as_uint(q.dx[1]), __float_as_uint(w3)));
-              __stcg(recs + 2 * r + 1,
-                     make_uint4(__float_as_uint(q.dxp[0]), __float_as_uint(q.dxp[1]),
-                                __float_as_uint(p3), __float_as_uint(coeff)));
-              continue;
-            }
+          for (int d = 0; d < D; ++d) {
+            const int f0 = shape_first_node<O>(q.ip[d], (real)q.dxp[d]);
+            const int f1 = shape_first_node<O>(q.i[d], (real)q.dx[d]);
+            word += (min(f0, f1) + ng) * (d == 0 ? 1 : (d == 1 ? G::WJ0 : G::WJ0 * G::WJ1));
+            cells |= ((unsigned)(q.i[d] - T0[d] + 64) << (8 * d)) |
+                     ((unsigned)(q.ip[d] - q.i[d] + 1) << (24 + 2 * d));
           }
+          const int region = unmoved ? 0 : 1;
+          unsigned  cls = (unsigned)word, row = 0;
+          for (int k = 0; k < 32; ++k, ++cls) {
+            cls &= 31u;
+            row = atomicAdd(&s_cnt[region][cls], 1u);
+            if (row < (unsigned)G::ROWS) break;
+          }
+          uint4*     r     = recs + (unmoved ? 0 : G::moved) + (size_t)(row * 32 + cls) * G::RECW;
+          const real coeff = wp * S.charge;
+          const unsigned z = D == 3 ? __float_as_uint(q.dx[2]) : 0u;
+          const unsigned y = D == 3 ? __float_as_uint(q.dxp[2]) : 0u;
+          if constexpr (sizeof(real) == 4) {
+            __stcg(r, make_uint4(cells, __float_as_uint(q.dx[0]), __float_as_uint(q.dx[1]),
+                                 D == 3 ? z : __float_as_uint((float)vp[2])));
+            __stcg(r + 1, make_uint4(__float_as_uint(q.dxp[0]), __float_as_uint(q.dxp[1]), y,
+                                     __float_as_uint((float)coeff)));
+          } else {
+            const long long cb = __double_as_longlong((double)coeff);
+            const long long vb = __double_as_longlong((double)vp[2]);
+            __stcg(r, make_uint4(cells, __float_as_uint(q.dx[0]), __float_as_uint(q.dx[1]), z));
+            __stcg(r + 1, make_uint4(__float_as_uint(q.dxp[0]), __float_as_uint(q.dxp[1]), y, 0u));
+            __stcg(r + 2, make_uint4((unsigned)cb, (unsigned)(cb >> 32), (unsigned)vb,
+                                     (unsigned)(vb >> 32)));
+          }
+        } else {
+          if (fixed)
+            deposit_particle<D, O, real, true>(q, wp, S.charge, a.inv_dt, a.dx, ng, nullptr,
+                                               add_fixed);
+          else
+            deposit_particle<D, O, real, true>(q, wp, S.charge, a.inv_dt, a.dx, ng, nullptr,
+                                               add_real);
         }
       }
-      deposit_particle<D, O, real>(q, wp, S.charge, a.inv_dt, a.dx, ng, nullptr, add);
-    }
-  }
-  __syncthreads();
-  if constexpr (G::STAGE) {
-    // the recorded particles, 32 per warp; the record's coefficient is the
-    // product weight * charge that the direct deposit forms, times charge 1
-    if (recs) {
-      const int nrec = min((int)s_nrec, a.st.cap);
-      unsigned* Jc   = Jw + (G::COPIES == 2 ? (int)(threadIdx.x & 1) * G::COPY : 0);
-      auto      add  = [&](int i, int j, int k, int c, real v) {
-        const int e = jb + i + j * G::WJ0 + k * (G::WJ0 * G::WJ1) + c * G::NJ;
-        if (fixed) FA::add(Jc + e, G::PLANE, v);
-        else       atomicAdd(Jr + e, v);
-      };
-      for (int r = threadIdx.x; r < nrec; r += NT) {
-        const uint4 u0 = __ldcg(recs + 2 * r), u1 = __ldcg(recs + 2 * r + 1);
-        Prtl<real>  q;
-        const float dx[3]  = { __uint_as_float(u0.y), __uint_as_float(u0.z), __uint_as_float(u0.w) };
-        const float dxp[3] = { __uint_as_float(u1.x), __uint_as_float(u1.y), __uint_as_float(u1.z) };
-        const real  vp[3]  = { 0, 0, D == 2 ? (real)dx[2] : (real)0 };
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          q.i[d]   = (int)((u0.x >> (8 * d)) & 255u) - 64 + T0[d];
-          q.ip[d]  = q.i[d] + (int)((u0.x >> (24 + 2 * d)) & 3u) - 1;
-          q.dx[d]  = dx[d];
-          q.dxp[d] = dxp[d];
-        }
-        deposit_with_velocity<D, O, real>(q, vp, (real)__uint_as_float(u1.w), (real)1, a.inv_dt,
-                                          ng, nullptr, add);
-        // Lanes 4m..4m+3 have read the four records of one 128-byte line and
-        // used them: the line is dropped from L2 unwritten, so the records
-        // cost no DRAM traffic (the next CTA on this buffer writes before it
-        // reads)
-        const int      base = r - (int)(threadIdx.x & 31);
-        const unsigned m    = nrec - base >= 32 ? 0xffffffffu : (1u << (nrec - base)) - 1u;
-        __syncwarp(m);
-        if ((r & 3) == 0) discard_l2_line(recs + 2 * r);
-      }
+      if (p0 < hi) break;  // the chunk is full
+      if (++s < a.nsp) p0 = a.s[s].tile_start[t];
     }
     __syncthreads();
-    if (threadIdx.x == 0 && slot >= 0) atomicExch(a.st.claim + slot, 0u);
+    if constexpr (REC) {
+      // a warp per row of records; a record's coefficient is the product
+      // weight * charge that the direct deposit forms, times charge 1
+      auto drain = [&](auto unmoved, const auto& add) {
+        constexpr bool UNMOVED = decltype(unmoved)::value;
+        const unsigned mine    = min(s_cnt[UNMOVED ? 0 : 1][lane], (unsigned)G::ROWS);
+        const int      rows    = (int)__reduce_max_sync(0xffffffffu, mine);
+        uint4*         first   = recs + (UNMOVED ? 0 : G::moved);
+        for (int row = wid; row < rows; row += NT / 32) {
+          uint4* line = first + (size_t)row * (32 * G::RECW);
+          if (row < (int)mine) {
+            const uint4* r  = line + lane * G::RECW;
+            const uint4  u0 = __ldcg(r), u1 = __ldcg(r + 1);
+            Prtl<real>   q;
+            const float dx[3]  = { __uint_as_float(u0.y), __uint_as_float(u0.z), __uint_as_float(u0.w) };
+            const float dxp[3] = { __uint_as_float(u1.x), __uint_as_float(u1.y), __uint_as_float(u1.z) };
+            real        vp[3]  = { 0, 0, 0 }, coeff;
+            if constexpr (sizeof(real) == 4) {
+              coeff = __uint_as_float(u1.w);
+              vp[2] = D == 2 ? dx[2] : 0.f;
+            } else {
+              const uint4 u2 = __ldcg(r + 2);
+              coeff = __hiloint2double((int)u2.y, (int)u2.x);
+              vp[2] = __hiloint2double((int)u2.w, (int)u2.z);
+            }
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              q.i[d]   = (int)((u0.x >> (8 * d)) & 255u) - 64 + T0[d];
+              q.ip[d]  = q.i[d] + (int)((u0.x >> (24 + 2 * d)) & 3u) - 1;
+              q.dx[d]  = dx[d];
+              q.dxp[d] = dxp[d];
+            }
+            deposit_with_velocity<D, O, real, UNMOVED ? BOX_UNMOVED : BOX_FULL>(q, vp, coeff, (real)1, a.inv_dt, ng, nullptr,
+                                                       add);
+          }
+          // the row has been used: its lines are dropped from L2 unwritten,
+          // so the records cost no DRAM traffic (a line is written again
+          // before it is read again)
+          __syncwarp();
+          if (lane < 4 * G::RECW) discard_l2_line((const char*)line + 128 * lane);
+        }
+      };
+      if (fixed) {
+        if constexpr (G::REC_ALL) drain(std::true_type{}, add_fixed);
+        drain(std::false_type{}, add_fixed);
+      } else {
+        if constexpr (G::REC_ALL) drain(std::true_type{}, add_real);
+        drain(std::false_type{}, add_real);
+      }
+      __syncthreads();
+      if (threadIdx.x < 64) (&s_cnt[0][0])[threadIdx.x] = 0u;
+    }
+    if (s >= a.nsp) break;
+    __syncthreads();
+  }
+  if constexpr (REC) {
+    if (threadIdx.x == 0) atomicExch(a.st.claim + s_slot, 0u);
   }
 
   // 3. flush the J window (periodic images folded onto active cells)
@@ -654,17 +731,8 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
     real      v = 0;
     long long units = 0;  // the entry in global units (exact accumulator)
     if (fixed) {
-      long long t = 0;
-      bool      any = false;
-#pragma unroll
-      for (int k = 0; k < G::COPIES; ++k) {
-        const unsigned* wk = Jw + k * G::COPY + idx;
-        if (FA::nonzero(wk, G::PLANE)) {
-          any = true;
-          t += FA::total(wk, G::PLANE);
-        }
-      }
-      if (!any) continue;
+      if (!FA::nonzero(Jw + idx, G::PLANE)) continue;
+      const long long t = FA::total(Jw + idx, G::PLANE);
       if (global_unit) units = (long long)((unsigned long long)t << (a.fj.bits - b));
       else             v = FA::to_real(t, unscale);
     } else {
@@ -706,6 +774,11 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
 
 template <int D, int O, typename real>
 cudaError_t launch_push_deposit_tiled(const TiledArgs<real>& a, cudaStream_t s);
+
+// 16-byte words of one record buffer and the number of buffers (the CTAs that
+// can be resident at once); no buffers (0, 0) where none are used
+template <int D, int O, typename real>
+cudaError_t deposit_record_words(size_t* words, int* slots);
 
 // tile shape of a build, for the host (sort key and tile count)
 void tile_shape(int dim, int real_bytes, int order, int out[3]);
