@@ -61,9 +61,14 @@ struct Philox4x32 {
     if (++ctr[0] == 0u) ++ctr[1];
     used = 0;
   }
+  // the block's four words in turn, picked by selects: an indexed buf would
+  // live in local memory
   __device__ uint32_t next() {
     if (used == 4) block();
-    return buf[used++];
+    const uint32_t lo = used & 1 ? buf[1] : buf[0], hi = used & 1 ? buf[3] : buf[2];
+    const uint32_t r  = used & 2 ? hi : lo;
+    ++used;
+    return r;
   }
 };
 

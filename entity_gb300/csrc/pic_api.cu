@@ -930,15 +930,18 @@ int pic_sort(pic_ctx* c, pic_species* sp, uint32_t flags, int64_t* npart_out, vo
   if (cells >= ((int64_t)1 << 31) - 2) return PIC_ERR_UNSUPPORTED;
   // any sort moves particles: the previous tile binning no longer holds
   if (SpeciesBins* b = find_bins(c, sp->index, false)) b->valid = false;
-  // scratch layout (8-byte aligned pieces)
-  auto          al   = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t  b_key = al(4 * np), b_rank = al(4 * np), b_dead = al(np), b_drank = al(4 * np);
-  const size_t  b_cnt = al(4 * (nbins + 1)), b_off = al(8 * (nbins + 1)), b_perm = al(4 * np);
-  const size_t  b_ptmp = al(4 * np), b_big = al(4 * nbins), b_nbig = al(4);
-  const size_t  rb     = (size_t)g.real_bytes;
+  // scratch layout (256-byte aligned pieces)
+  auto          al      = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const int64_t nblocks = (np + pic::kSortBlock - 1) / pic::kSortBlock;
+  const size_t  b_rank = al(4 * np), b_perm = al(4 * np), b_dead = al(4 * nblocks);
+  const size_t  b_cnt = al(4 * (nbins + 1)), b_off = al(8 * (nbins + 1));
+  const size_t  b_big = al(4 * (np / pic::kBigBin + 1)), b_nbig = al(4);
+  const size_t  rb    = (size_t)g.real_bytes;
+  const bool    prev  = !skip_prev;
   // the arrays a sort moves (Particles::SortSpatially and RemoveDead,
-  // particles_sort.cpp:103-253): the state, then phi and every payload
-  // column; in batches of up to kMaxSortArrays
+  // particles_sort.cpp:103-253): the state, as records; phi and every payload
+  // column, gathered through the permutation in batches of up to
+  // kMaxSortArrays. Without room for the records the state is gathered too.
   struct Moved {
     void*   arr;
     int     esz;
@@ -948,101 +951,107 @@ int pic_sort(pic_ctx* c, pic_species* sp, uint32_t flags, int64_t* npart_out, vo
   auto add = [&](void* arr, int esz, int64_t stride = 1) {
     if (arr) mv.push_back({ arr, esz, stride });
   };
-  add(sp->i1, 4), add(sp->i2, 4), add(sp->dx1, 4), add(sp->dx2, 4);
-  if (g.dim == 3) add(sp->i3, 4), add(sp->dx3, 4);
-  if (!skip_prev) {
-    add(sp->i1_prev, 4), add(sp->i2_prev, 4), add(sp->dx1_prev, 4), add(sp->dx2_prev, 4);
-    if (g.dim == 3) add(sp->i3_prev, 4), add(sp->dx3_prev, 4);
-  }
-  add(sp->ux1, (int)rb), add(sp->ux2, (int)rb), add(sp->ux3, (int)rb), add(sp->weight, (int)rb);
-  add(sp->tag, 2);
   add(sp->phi, (int)rb);
   for (int k = 0; k < sp->npld_r; ++k)
     add((char*)sp->pld_r + (size_t)k * sp->pld_r_stride[1] * rb, (int)rb, sp->pld_r_stride[0]);
   // integer payloads are npart_t, 32-bit (global.h:385)
   for (int k = 0; k < sp->npld_i; ++k)
     add((char*)sp->pld_i + (size_t)k * sp->pld_i_stride[1] * 4, 4, sp->pld_i_stride[0]);
-  // every array of a batch gets its own staging area when the context can
-  // hold them (one gather, one copy back per batch); otherwise they go in
-  // turn through one
-  size_t b_all = 0;
+  // the extra arrays of a batch get their own staging areas (one gather, one
+  // copy back per batch); when the context cannot hold all that, every array
+  // goes in turn through one
+  const size_t b_rec = al((size_t)np * 16 * pic::sort_record_words(g.dim, g.real_bytes, prev));
+  size_t       b_all = 0;
   for (size_t k = 0; k < mv.size() && k < (size_t)pic::kMaxSortArrays; ++k)
     b_all += al((size_t)np * mv[k].esz);
-  const size_t b_big_elem = al(np * 8);
-  const size_t b_one = b_big_elem;
-  const size_t  fixed_need = b_key + b_rank + b_dead + b_drank + b_cnt + b_off + b_perm + b_ptmp +
-                            b_big + b_nbig;
-  bool          apart      = true;
-  if (fixed_need + b_all > c->sort_bytes) {
+  const size_t b_one      = al(np * 8);
+  // with records the permutation is needed for extra arrays only
+  const size_t fixed_need = b_rank + 2 * b_dead + b_cnt + b_off + b_big + b_nbig;
+  const size_t rec_need   = fixed_need + b_rec + (mv.empty() ? 0 : b_perm + b_all);
+  const size_t one_need   = fixed_need + 2 * b_perm + b_one;
+  bool         records    = true;
+  if (rec_need > c->sort_bytes) {
     if (c->sort_buf) cudaFree(c->sort_buf);
     c->sort_buf   = nullptr;
     c->sort_bytes = 0;
-    if (cudaMalloc(&c->sort_buf, fixed_need + b_all) == cudaSuccess) {
-      c->sort_bytes = fixed_need + b_all;
+    if (cudaMalloc(&c->sort_buf, rec_need) == cudaSuccess) {
+      c->sort_bytes = rec_need;
     } else {
       cudaGetLastError();  // the failed allocation leaves no sticky error
-      apart = false;
-      if (fixed_need + b_one > c->sort_bytes) {
-        if (cudaMalloc(&c->sort_buf, fixed_need + b_one) != cudaSuccess) return PIC_ERR_NOMEM;
-        c->sort_bytes = fixed_need + b_one;
-      }
+      records = false;
+      if (cudaMalloc(&c->sort_buf, one_need) != cudaSuccess) return PIC_ERR_NOMEM;
+      c->sort_bytes = one_need;
     }
   }
-  char*         base = (char*)c->sort_buf;
-  pic::SortArgs a;
-  a.i1 = sp->i1;
-  a.i2 = sp->i2;
-  a.i3 = sp->i3;
-  a.tag = sp->tag;
-  a.npart = np;
-  a.dim = g.dim;
-  a.n[0] = g.n[0];
-  a.n[1] = g.n[1];
-  a.n[2] = g.n[2];
-  a.spatial = spatial ? 1 : 0;
-  a.tiled   = tiled ? 1 : 0;
+  if (!records) {
+    add(sp->i1, 4), add(sp->i2, 4), add(sp->dx1, 4), add(sp->dx2, 4);
+    if (g.dim == 3) add(sp->i3, 4), add(sp->dx3, 4);
+    if (prev) {
+      add(sp->i1_prev, 4), add(sp->i2_prev, 4), add(sp->dx1_prev, 4), add(sp->dx2_prev, 4);
+      if (g.dim == 3) add(sp->i3_prev, 4), add(sp->dx3_prev, 4);
+    }
+    add(sp->ux1, (int)rb), add(sp->ux2, (int)rb), add(sp->ux3, (int)rb), add(sp->weight, (int)rb);
+    add(sp->tag, 2);
+  }
+  char* base = (char*)c->sort_buf;
+  auto  take = [&](size_t b) {
+    char* q = base;
+    base += b;
+    return q;
+  };
+  pic::SortArgs a{};
+  int32_t* const ii[3] = { sp->i1, sp->i2, sp->i3 };
+  int32_t* const pp[3] = { sp->i1_prev, sp->i2_prev, sp->i3_prev };
+  float* const   xx[3] = { sp->dx1, sp->dx2, sp->dx3 };
+  float* const   yy[3] = { sp->dx1_prev, sp->dx2_prev, sp->dx3_prev };
+  void* const    uu[4] = { sp->ux1, sp->ux2, sp->ux3, sp->weight };
   for (int d = 0; d < 3; ++d) {
-    a.tile[d]   = ts[d];
+    a.i[d] = ii[d], a.ip[d] = pp[d], a.dx[d] = xx[d], a.dxp[d] = yy[d];
+    a.n[d]      = g.n[d];
     a.ntiles[d] = nt[d];
+    while ((1 << a.tile_log[d]) < ts[d]) ++a.tile_log[d];
+    if ((1 << a.tile_log[d]) != ts[d]) return PIC_ERR_UNSUPPORTED;  // tile sides are powers of two
   }
-  a.dead_bin = (int32_t)cells;
-  a.key = (int32_t*)base;
-  base += b_key;
-  a.rank = (int32_t*)base;
-  base += b_rank;
-  a.is_dead = (uint8_t*)base;
-  base += b_dead;
-  a.dead_rank = (int32_t*)base;
-  base += b_drank;
-  a.count = (int32_t*)base;
-  base += b_cnt;
-  a.off = (int64_t*)base;
-  base += b_off;
-  a.perm = (int32_t*)base;
-  base += b_perm;
-  a.perm_tmp = (int32_t*)base;
-  base += b_ptmp;
-  a.big = (int32_t*)base;
-  base += b_big;
-  a.nbig = (int32_t*)base;
-  base += b_nbig;
-  a.err = c->d_err;
+  for (int k = 0; k < 4; ++k) a.u[k] = uu[k];
+  a.tag        = sp->tag;
+  a.real_bytes = g.real_bytes;
+  a.prev       = prev;
+  a.npart      = np;
+  a.dim        = g.dim;
+  a.spatial    = spatial ? 1 : 0;
+  a.tiled      = tiled ? 1 : 0;
+  a.dead_bin   = (int32_t)cells;
+  a.rank       = (int32_t*)take(b_rank);
+  a.dead_off   = (int32_t*)take(b_dead);
+  a.dead_cnt   = (int32_t*)take(b_dead);
+  a.count      = (int32_t*)take(b_cnt);
+  a.off        = (int64_t*)take(b_off);
+  a.big        = (int32_t*)take(b_big);
+  a.nbig       = (int32_t*)take(b_nbig);
+  a.err        = c->d_err;
+  a.rec        = records ? (uint4*)take(b_rec) : nullptr;
+  a.perm       = records ? nullptr : (int32_t*)take(b_perm);
+  a.perm2      = mv.empty() ? nullptr : (int32_t*)take(b_perm);
 
-  cudaError_t e = pic::sort_build_perm(a, s);
+  cudaError_t e = pic::sort_scatter(a, s);
   if (e != cudaSuccess) return PIC_ERR_CUDA;
-  for (size_t k0 = 0; k0 < mv.size(); k0 += pic::kMaxSortArrays) {
-    pic::GatherSet gs;
-    char*          t = base;
-    for (size_t k = k0; k < mv.size() && gs.n < pic::kMaxSortArrays; ++k) {
-      gs.arr[gs.n]    = mv[k].arr;
-      gs.esz[gs.n]    = mv[k].esz;
-      gs.stride[gs.n] = mv[k].stride;
-      gs.tmp[gs.n]    = t;
-      if (apart) t += al((size_t)np * mv[k].esz);
-      ++gs.n;
+  if (!mv.empty()) {
+    if ((e = pic::sort_final_perm(a, s)) != cudaSuccess) return PIC_ERR_CUDA;
+    for (size_t k0 = 0; k0 < mv.size(); k0 += pic::kMaxSortArrays) {
+      pic::GatherSet gs;
+      char*          t = base;
+      for (size_t k = k0; k < mv.size() && gs.n < pic::kMaxSortArrays; ++k) {
+        gs.arr[gs.n]    = mv[k].arr;
+        gs.esz[gs.n]    = mv[k].esz;
+        gs.stride[gs.n] = mv[k].stride;
+        gs.tmp[gs.n]    = t;
+        if (records) t += al((size_t)np * mv[k].esz);
+        ++gs.n;
+      }
+      if ((e = pic::sort_apply_all(gs, a.perm2, np, s)) != cudaSuccess) return PIC_ERR_CUDA;
     }
-    if ((e = pic::sort_apply_all(gs, a.perm, np, s)) != cudaSuccess) return PIC_ERR_CUDA;
   }
+  if (records && (e = pic::sort_unpack(a, s)) != cudaSuccess) return PIC_ERR_CUDA;
   if (remove_dead) {
     // particles_sort.cpp:175-191: alive tags on the front, dead on the tail
     if ((e = pic::set_tags_after_removal(sp->tag, np, a.count + a.dead_bin, s)) != cudaSuccess)

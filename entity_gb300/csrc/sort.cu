@@ -7,17 +7,23 @@
 // (ascending original index inside every cell), which is one of the orders
 // the reference may produce, and is deterministic:
 //   1. key per particle (PositionToTileIndex, src/global/utils/sorting.h:
-//      119-135: (i1*n2 + i2)*n3 + i3; dead -> last bin) and an atomic count
-//      per bin whose return value is a provisional rank;
-//   2. exclusive scan of the counts -> bin offsets;
-//   3. scatter of indices; dead particles get their rank from a scan so the
-//      (possibly huge) dead bin is placed in order directly;
-//   4. every alive bin's index list is sorted ascending (one thread per bin up
-//      to 32 entries, one block per larger bin);
-//   5. every particle array is gathered through the permutation and copied
-//      back.
+//      119-135: (i1*n2 + i2)*n3 + i3; dead -> last bin) and a count per bin;
+//      the counting atomics (one per group of a warp's lanes with one key)
+//      return each particle's place in its bin, in arrival order;
+//   2. exclusive scan of the counts -> bin offsets; the dead are counted per
+//      block of particles, whose scan places them in order;
+//   3. every particle's arrays are packed into one record at its place;
+//   4. a pass over the records writes them back into the arrays, each bin in
+//      ascending original index: a particle's place in its bin is the number
+//      of smaller indices there (bins above kBigBin are sorted first).
+// Packed records instead of one gather per array: a random particle order
+// touches two 32-byte sectors per particle instead of one per array (11 in
+// FP32 3D), and nothing is copied back. 2 x 16.8 M particles in random order
+// (128^3 cells, with the injection) went from 9.45 to 4.19 ms.
 // Nothing here synchronises with the host; the dead count stays on the
 // device until the caller reads it.
+#include <type_traits>
+
 #include <cuda_runtime.h>
 
 #include "sort.cuh"
@@ -133,12 +139,8 @@ cudaError_t exclusive_scan(const Tin* in, int64_t n, T* out, ScanScratch<T>& scr
 
 template cudaError_t exclusive_scan<int32_t, int64_t>(const int32_t*, int64_t, int64_t*,
                                                       ScanScratch<int64_t>&, cudaStream_t);
-template cudaError_t exclusive_scan<uint8_t, int64_t>(const uint8_t*, int64_t, int64_t*,
-                                                      ScanScratch<int64_t>&, cudaStream_t);
 template cudaError_t exclusive_scan<int64_t, int64_t>(const int64_t*, int64_t, int64_t*,
                                                       ScanScratch<int64_t>&, cudaStream_t);
-template cudaError_t exclusive_scan<uint8_t, int32_t>(const uint8_t*, int64_t, int32_t*,
-                                                      ScanScratch<int32_t>&, cudaStream_t);
 template cudaError_t exclusive_scan<int32_t, int32_t>(const int32_t*, int64_t, int32_t*,
                                                       ScanScratch<int32_t>&, cudaStream_t);
 
@@ -152,102 +154,309 @@ __device__ __forceinline__ int tile_row_slot(int lx, int tx) {
   return (lx & 1) ? (tx + 1) / 2 + lx / 2 : lx / 2;
 }
 
-// 1. keys + counts + provisional rank
-__global__ void k_keys(SortArgs a) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.npart; p += stride) {
-    const short tag = a.tag[p];
-    int32_t     key;
-    if (tag != PIC_TAG_ALIVE) {
-      key = a.dead_bin;
-    } else if (!a.spatial) {
-      key = 0;
-    } else {
-      const int i1 = a.i1[p], i2 = a.i2[p], i3 = a.dim == 3 ? a.i3[p] : 0;
-      const bool ok = (i1 >= 0 && i1 < a.n[0] && i2 >= 0 && i2 < a.n[1] &&
-                       (a.dim == 2 || (i3 >= 0 && i3 < a.n[2])));
-      if (!ok) {
-        atomicAdd(a.err + ERR_OUT_OF_GRID, 1ull);
-        key = a.dead_bin;  // kept after the alive particles, tag untouched
-      } else if (a.tiled) {
-        const int tx = i1 / a.tile[0], ty = i2 / a.tile[1], tz = i3 / a.tile[2];
-        const int lx = i1 - tx * a.tile[0], ly = i2 - ty * a.tile[1], lz = i3 - tz * a.tile[2];
-        const int t  = (tz * a.ntiles[1] + ty) * a.ntiles[0] + tx;
-        key = (t * a.tile[2] + lz) * (a.tile[0] * a.tile[1]) + ly * a.tile[0] +
-              tile_row_slot(lx, a.tile[0]);
-      } else if (a.dim == 2) {
-        key = i1 * a.n[1] + i2;
+// the bin of one particle; ok = false for a live particle outside the grid
+// (kept with the dead, tag untouched)
+__device__ __forceinline__ int32_t sort_key(const SortArgs& a, short tag, int i1, int i2, int i3,
+                                            bool& ok) {
+  ok = true;
+  if (tag != PIC_TAG_ALIVE) return a.dead_bin;
+  if (!a.spatial) return 0;
+  ok = i1 >= 0 && i1 < a.n[0] && i2 >= 0 && i2 < a.n[1] && (a.dim == 2 || (i3 >= 0 && i3 < a.n[2]));
+  if (!ok) return a.dead_bin;
+  if (a.tiled) {
+    const int tx = i1 >> a.tile_log[0], ty = i2 >> a.tile_log[1], tz = i3 >> a.tile_log[2];
+    const int sx = 1 << a.tile_log[0];
+    const int lx = i1 & (sx - 1), ly = i2 & ((1 << a.tile_log[1]) - 1),
+              lz = i3 & ((1 << a.tile_log[2]) - 1);
+    const int t  = (tz * a.ntiles[1] + ty) * a.ntiles[0] + tx;
+    return (((((t << a.tile_log[2]) + lz) << a.tile_log[1]) + ly) << a.tile_log[0]) +
+           tile_row_slot(lx, sx);
+  }
+  return a.dim == 2 ? i1 * a.n[1] + i2 : (i1 * a.n[1] + i2) * a.n[2] + i3;
+}
+
+__device__ __forceinline__ int32_t sort_key_at(const SortArgs& a, int64_t p, bool& ok) {
+  return sort_key(a, a.tag[p], a.i[0][p], a.i[1][p], a.dim == 3 ? a.i[2][p] : 0, ok);
+}
+
+// 1. places within the bins and counts; the dead per block
+__global__ void __launch_bounds__(256) k_keys(SortArgs a) {
+  __shared__ int s_dead;
+  const int64_t  p0 = (int64_t)blockIdx.x * kSortBlock;
+  const int      lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) s_dead = 0;
+  __syncthreads();
+  int dead = 0;
+  for (int it = 0; it < kSortBlock / 256; ++it) {
+    const int64_t p   = p0 + it * 256 + threadIdx.x;
+    int32_t       key = -1;
+    bool          ok  = true;
+    if (p < a.npart) key = sort_key_at(a, p, ok);
+    if (!ok) atomicAdd(a.err + ERR_OUT_OF_GRID, 1ull);
+    dead += key == a.dead_bin;
+    if (!a.spatial) continue;
+    // one atomic for the lanes of a warp that share a bin
+    const unsigned peers  = __match_any_sync(0xffffffffu, key);
+    const int      leader = __ffs(peers) - 1, cnt = __popc(peers);
+    const bool     live   = key >= 0 && key != a.dead_bin;
+    int            base   = 0;
+    if (lane == leader && live) {
+      base = atomicAdd(a.count + key, cnt);
+      if (base <= kBigBin && base + cnt > kBigBin) a.big[atomicAdd(a.nbig, 1)] = key;
+    }
+    base = __shfl_sync(0xffffffffu, base, leader);
+    if (live) a.rank[p] = base + __popc(peers & ((1u << lane) - 1u));
+  }
+  dead = __reduce_add_sync(0xffffffffu, dead);
+  if (lane == 0 && dead) atomicAdd(&s_dead, dead);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.dead_cnt[blockIdx.x] = s_dead;
+    if (s_dead) atomicAdd(a.count + a.dead_bin, s_dead);
+    if (!a.spatial) {  // one bin of the living
+      const int64_t here = a.npart - p0 < kSortBlock ? a.npart - p0 : kSortBlock;
+      atomicAdd(a.count, (int)here - s_dead);
+    }
+  }
+}
+
+// one particle's arrays as 32-bit words: cells, offsets, [previous ones],
+// momenta and weight, tag, original index
+template <int D, int RW, bool PREV>
+struct SortRec {
+  static constexpr int DIM  = D;
+  static constexpr int DATA = (PREV ? 4 : 2) * D + 4 * RW + 1;  // words before the index
+  static constexpr int Q    = (DATA + 1 + 7) / 8 * 2;           // 16-byte words, whole 32-byte sectors
+  unsigned w[4 * Q];
+  __device__ __forceinline__ void load(const SortArgs& a, int64_t p) {
+    int k = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) w[k++] = (unsigned)a.i[d][p];
+#pragma unroll
+    for (int d = 0; d < D; ++d) w[k++] = __float_as_uint(a.dx[d][p]);
+    if constexpr (PREV) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) w[k++] = (unsigned)a.ip[d][p];
+#pragma unroll
+      for (int d = 0; d < D; ++d) w[k++] = __float_as_uint(a.dxp[d][p]);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if constexpr (RW == 1) {
+        w[k++] = ((const unsigned*)a.u[c])[p];
       } else {
-        key = (i1 * a.n[1] + i2) * a.n[2] + i3;
+        const uint2 v = ((const uint2*)a.u[c])[p];
+        w[k++] = v.x, w[k++] = v.y;
       }
     }
-    a.key[p]        = key;
-    a.is_dead[p]    = (uint8_t)(key == a.dead_bin);
-    a.rank[p]       = atomicAdd(a.count + key, 1);
+    w[k++] = (unsigned short)a.tag[p];
+    w[k++] = (unsigned)p;
+#pragma unroll
+    for (; k < 4 * Q; ++k) w[k] = 0u;
   }
-}
-
-// 3. scatter of particle indices into their bins
-__global__ void k_scatter(SortArgs a) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.npart; p += stride) {
-    const int32_t key = a.key[p];
-    int64_t       pos;
-    if (key == a.dead_bin) {
-      pos = a.off[key] + a.dead_rank[p];
-    } else if (!a.spatial) {
-      pos = p - a.dead_rank[p];  // alive before p, in order
-    } else {
-      pos = a.off[key] + a.rank[p];
+  __device__ __forceinline__ void store(const SortArgs& a, int64_t p) const {
+    int k = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) a.i[d][p] = (int)w[k++];
+#pragma unroll
+    for (int d = 0; d < D; ++d) a.dx[d][p] = __uint_as_float(w[k++]);
+    if constexpr (PREV) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) a.ip[d][p] = (int)w[k++];
+#pragma unroll
+      for (int d = 0; d < D; ++d) a.dxp[d][p] = __uint_as_float(w[k++]);
     }
-    a.perm[pos] = (int32_t)p;
-  }
-}
-
-// 4a. per-bin ascending order, small bins
-__global__ void k_fix_small(SortArgs a) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < a.dead_bin; b += stride) {
-    const int64_t lo = a.off[b], hi = a.off[b + 1];
-    const int64_t m  = hi - lo;
-    if (m <= 1) continue;
-    if (m > 32) {
-      const int slot = atomicAdd(a.nbig, 1);
-      a.big[slot]    = (int32_t)b;
-      continue;
-    }
-    int32_t v[32];
-    for (int q = 0; q < m; ++q) v[q] = a.perm[lo + q];
-    for (int q = 1; q < m; ++q) {
-      const int32_t x = v[q];
-      int           r = q - 1;
-      while (r >= 0 && v[r] > x) {
-        v[r + 1] = v[r];
-        --r;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if constexpr (RW == 1) {
+        ((unsigned*)a.u[c])[p] = w[k++];
+      } else {
+        ((uint2*)a.u[c])[p] = make_uint2(w[k], w[k + 1]);
+        k += 2;
       }
-      v[r + 1] = x;
     }
-    for (int q = 0; q < m; ++q) a.perm[lo + q] = v[q];
+    a.tag[p] = (int16_t)(uint16_t)w[k];
+  }
+  __device__ __forceinline__ short tag() const { return (short)(uint16_t)w[DATA - 1]; }
+  __device__ __forceinline__ int32_t index() const { return (int32_t)w[DATA]; }
+};
+// perm only (no records)
+struct NoRec {
+  static constexpr int Q = 1;
+};
+
+// 3. the records packed to their places (or, without records, the
+// permutation). A warp's records pass through shared memory, so that
+// consecutive lanes write one record's consecutive 16-byte words.
+template <typename R>
+__global__ void __launch_bounds__(256) k_scatter(SortArgs a) {
+  constexpr bool PACK = !std::is_same_v<R, NoRec>;
+  __shared__ uint4   s_rec[PACK ? 256 * R::Q : 1];
+  __shared__ int64_t s_pos[256];
+  __shared__ int     s_warp[8];
+  const int64_t p0 = (int64_t)blockIdx.x * kSortBlock;
+  const int     lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // dead particles before the block's next 256, and whether it holds any
+  int64_t    dead0    = a.dead_off[blockIdx.x];
+  const bool any_dead = a.dead_cnt[blockIdx.x] != 0;
+  for (int it = 0; it < kSortBlock / 256; ++it) {
+    const int64_t p = p0 + it * 256 + threadIdx.x;
+    if (p0 + it * 256 >= a.npart) break;  // the same for the whole block
+    int32_t key = -1;
+    bool    ok;
+    R       r;
+    if (p < a.npart) {
+      if constexpr (PACK) {
+        r.load(a, p);
+        key = sort_key(a, r.tag(), (int)r.w[0], (int)r.w[1], R::DIM == 3 ? (int)r.w[2] : 0, ok);
+      } else {
+        key = sort_key_at(a, p, ok);
+      }
+    }
+    const bool dead   = key == a.dead_bin;
+    int64_t    before = dead0;  // dead particles before p
+    if (any_dead) {
+      const unsigned ball = __ballot_sync(0xffffffffu, dead);
+      if (lane == 0) s_warp[wid] = __popc(ball);
+      __syncthreads();
+      int total = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        if (w < wid) before += s_warp[w];
+        total += s_warp[w];
+      }
+      before += __popc(ball & ((1u << lane) - 1u));
+      dead0 += total;
+      __syncthreads();
+    }
+    int64_t pos = -1;
+    if (key >= 0)
+      pos = dead ? a.off[key] + before : (a.spatial ? a.off[key] + a.rank[p] : p - before);
+    if constexpr (PACK) {
+      uint4* mine = s_rec + wid * (32 * R::Q);
+#pragma unroll
+      for (int q = 0; q < R::Q; ++q)
+        mine[lane * R::Q + q] =
+            make_uint4(r.w[4 * q], r.w[4 * q + 1], r.w[4 * q + 2], r.w[4 * q + 3]);
+      s_pos[threadIdx.x] = pos;
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < R::Q; ++q) {
+        const int     e = q * 32 + lane, t = e / R::Q;
+        const int64_t d = s_pos[wid * 32 + t];
+        if (d >= 0) a.rec[d * R::Q + e % R::Q] = mine[e];
+      }
+      __syncwarp();
+    } else if (pos >= 0) {
+      a.perm[pos] = (int32_t)p;
+    }
   }
 }
 
-// 4b. large bins: rank by counting (O(m^2 / threads)); blocks stride over
-// the bins the small-bin pass listed, whose number only the device knows
+// the original index of the particle at place p after the scatter
+template <typename R>
+__device__ __forceinline__ int32_t index_at(const SortArgs& a, int64_t p) {
+  if constexpr (std::is_same_v<R, NoRec>) return a.perm[p];
+  else return (int32_t)((const unsigned*)a.rec)[p * (4 * R::Q) + R::DATA];
+}
+
+// bins above kBigBin: their indices put in order in a.rank (free after the
+// scatter) by rank counting (O(m^2 / threads)); blocks stride over the bins
+// the counting listed, whose number only the device knows
+template <typename R>
 __global__ void k_fix_big(SortArgs a) {
   const int nbig = *a.nbig;
   for (int bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
     const int     b  = a.big[bi];
     const int64_t lo = a.off[b], hi = a.off[b + 1];
-    const int64_t m  = hi - lo;
-    for (int64_t q = threadIdx.x; q < m; q += blockDim.x) {
-      const int32_t x = a.perm[lo + q];
-      int64_t       r = 0;
-      for (int64_t z = 0; z < m; ++z) r += (a.perm[lo + z] < x);
-      a.perm_tmp[lo + r] = x;
+    for (int64_t q = lo + threadIdx.x; q < hi; q += blockDim.x) {
+      const int32_t x = index_at<R>(a, q);
+      int64_t       r = lo;
+      for (int64_t z = lo; z < hi; ++z) r += index_at<R>(a, z) < x;
+      a.rank[r] = x;
     }
-    __syncthreads();
-    for (int64_t q = threadIdx.x; q < m; q += blockDim.x) a.perm[lo + q] = a.perm_tmp[lo + q];
-    __syncthreads();
+  }
+}
+
+// place of index x in a big bin [lo, hi), whose indices are in order in a.rank
+__device__ __forceinline__ int64_t big_place(const SortArgs& a, int64_t lo, int64_t hi, int32_t x) {
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (a.rank[mid] < x) lo = mid + 1;
+    else                 hi = mid;
+  }
+  return lo;
+}
+
+// 4. records back into the arrays, each at the place that the number of
+// smaller indices in its bin gives it (the dead and a plain compaction are in
+// order as they are). A block's records are consecutive: they are read 16
+// bytes per thread and handed over in shared memory, where most of a bin's
+// indices are found too
+template <typename R>
+__global__ void __launch_bounds__(256) k_unpack(SortArgs a) {
+  __shared__ uint4   s_rec[256 * R::Q];
+  __shared__ int32_t s_idx[256];
+  const int64_t p0 = (int64_t)blockIdx.x * 256;
+  const int     n  = (int)(a.npart - p0 < 256 ? a.npart - p0 : 256);
+#pragma unroll
+  for (int q = 0; q < R::Q; ++q) {
+    const int e = q * 256 + (int)threadIdx.x;
+    if (e < n * R::Q) s_rec[e] = __ldcs(a.rec + p0 * R::Q + e);
+  }
+  __syncthreads();
+  R r;
+#pragma unroll
+  for (int q = 0; q < R::Q; ++q) {
+    const uint4 v = s_rec[threadIdx.x * R::Q + q];
+    r.w[4 * q] = v.x, r.w[4 * q + 1] = v.y, r.w[4 * q + 2] = v.z, r.w[4 * q + 3] = v.w;
+  }
+  const int32_t x    = r.index();
+  s_idx[threadIdx.x] = x;
+  __syncthreads();
+  if ((int)threadIdx.x >= n) return;
+  bool          ok;
+  const int32_t key =
+    sort_key(a, r.tag(), (int)r.w[0], (int)r.w[1], R::DIM == 3 ? (int)r.w[2] : 0, ok);
+  int64_t place = p0 + threadIdx.x;
+  if (a.spatial && key != a.dead_bin) {
+    const int64_t lo = a.off[key], hi = a.off[key + 1];
+    if (hi - lo > kBigBin) {
+      place = big_place(a, lo, hi, x);
+    } else {
+      // the bin's part in this block, then what lies before and after it
+      const int b0 = (int)(lo > p0 ? lo - p0 : 0), b1 = (int)(hi < p0 + n ? hi - p0 : n);
+      int       smaller = 0;
+#pragma unroll 4
+      for (int z = b0; z < b1; ++z) smaller += s_idx[z] < x;
+      for (int64_t z = lo; z < p0; ++z) smaller += index_at<R>(a, z) < x;
+      for (int64_t z = p0 + n; z < hi; ++z) smaller += index_at<R>(a, z) < x;
+      place = lo + smaller;
+    }
+  }
+  r.store(a, place);
+}
+
+// the permutation (new index -> old index) into a.perm2, from the particle
+// arrays as they were
+template <typename R>
+__global__ void k_final_perm(SortArgs a) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.npart; p += stride) {
+    const int32_t x = index_at<R>(a, p);
+    bool          ok;
+    const int32_t key   = sort_key_at(a, x, ok);
+    int64_t       place = p;
+    if (a.spatial && key != a.dead_bin) {
+      const int64_t lo = a.off[key], hi = a.off[key + 1];
+      if (hi - lo > kBigBin) {
+        place = big_place(a, lo, hi, x);
+      } else {
+        place = lo;
+        for (int64_t z = lo; z < hi; ++z) place += index_at<R>(a, z) < x;
+      }
+    }
+    a.perm2[place] = x;
   }
 }
 
@@ -281,34 +490,75 @@ dim3 grid_n(int64_t n) {
 
 }  // namespace
 
-cudaError_t sort_build_perm(SortArgs a, cudaStream_t s) {
-  cudaError_t e;
-  const int64_t nbins = (int64_t)a.dead_bin + 1;
-  e = cudaMemsetAsync(a.count, 0, sizeof(int32_t) * (nbins + 1), s);
-  if (e != cudaSuccess) return e;
-  PIC_KL(k_keys<<<grid_n(a.npart), 256, 0, s>>>(a));
+namespace {
+// calls f.operator()<D, RW, PREV>() for the species' layout
+template <typename F>
+cudaError_t by_layout(int dim, int real_bytes, bool prev, F&& f) {
+  const int rw = real_bytes / 4;
+#define PIC_SR(DD, RR, PP) \
+  if (dim == DD && rw == RR && prev == PP) return f(SortRec<DD, RR, PP>{});
+  PIC_SR(2, 1, false)
+  PIC_SR(2, 1, true)
+  PIC_SR(2, 2, false)
+  PIC_SR(2, 2, true)
+  PIC_SR(3, 1, false)
+  PIC_SR(3, 1, true)
+  PIC_SR(3, 2, false)
+  PIC_SR(3, 2, true)
+#undef PIC_SR
+  return cudaErrorInvalidValue;
+}
+template <typename F>
+cudaError_t with_layout(const SortArgs& a, F&& f) {
+  return a.rec ? by_layout(a.dim, a.real_bytes, a.prev, f) : f(NoRec{});
+}
+}  // namespace
+
+int sort_record_words(int dim, int real_bytes, bool prev) {
+  int q = 0;
+  by_layout(dim, real_bytes, prev, [&](auto r) {
+    q = decltype(r)::Q;
+    return cudaSuccess;
+  });
+  return q;
+}
+
+cudaError_t sort_scatter(const SortArgs& a, cudaStream_t s) {
+  cudaError_t   e;
+  const int64_t nbins  = (int64_t)a.dead_bin + 1;
+  const int64_t blocks = (a.npart + kSortBlock - 1) / kSortBlock;
+  if ((e = cudaMemsetAsync(a.count, 0, sizeof(int32_t) * (nbins + 1), s)) != cudaSuccess) return e;
+  if ((e = cudaMemsetAsync(a.nbig, 0, sizeof(int32_t), s)) != cudaSuccess) return e;
+  PIC_KL(k_keys<<<(unsigned)blocks, 256, 0, s>>>(a));
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   ScanScratch<int64_t> scr;
   e = exclusive_scan<int32_t, int64_t>(a.count, nbins + 1, a.off, scr, s);
   scr.release(s);
   if (e != cudaSuccess) return e;
-  // the rank of every particle among the dead (and, for the alive-only
-  // compaction, the number of dead before it): one scan, whatever the count
   ScanScratch<int32_t> scr2;
-  e = exclusive_scan<uint8_t, int32_t>(a.is_dead, a.npart, a.dead_rank, scr2, s);
+  e = exclusive_scan<int32_t, int32_t>(a.dead_cnt, blocks, a.dead_off, scr2, s);
   scr2.release(s);
   if (e != cudaSuccess) return e;
-  PIC_KL(k_scatter<<<grid_n(a.npart), 256, 0, s>>>(a));
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (a.spatial && a.dead_bin > 0) {
-    e = cudaMemsetAsync(a.nbig, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return e;
-    PIC_KL(k_fix_small<<<grid_n(a.dead_bin), 256, 0, s>>>(a));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    PIC_KL(k_fix_big<<<pic::sm_count() * 2, 256, 0, s>>>(a));
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  return with_layout(a, [&](auto r) {
+    using R = decltype(r);
+    PIC_KL(k_scatter<R><<<(unsigned)blocks, 256, 0, s>>>(a));
+    if (a.spatial && a.npart > kBigBin) PIC_KL(k_fix_big<R><<<pic::sm_count() * 2, 256, 0, s>>>(a));
+    return cudaGetLastError();
+  });
+}
+
+cudaError_t sort_unpack(const SortArgs& a, cudaStream_t s) {
+  return by_layout(a.dim, a.real_bytes, a.prev, [&](auto r) {
+    PIC_KL(k_unpack<decltype(r)><<<(unsigned)((a.npart + 255) / 256), 256, 0, s>>>(a));
+    return cudaGetLastError();
+  });
+}
+
+cudaError_t sort_final_perm(const SortArgs& a, cudaStream_t s) {
+  return with_layout(a, [&](auto r) {
+    PIC_KL(k_final_perm<decltype(r)><<<grid_n(a.npart), 256, 0, s>>>(a));
+    return cudaGetLastError();
+  });
 }
 
 namespace {

@@ -33,35 +33,54 @@ struct ScanScratch {
 template <typename Tin, typename T>
 cudaError_t exclusive_scan(const Tin* in, int64_t n, T* out, ScanScratch<T>& scr, cudaStream_t s);
 
+// particles per block of the key and scatter passes, in index order (the dead
+// of a block are counted together)
+constexpr int kSortBlock = 2048;
+// bins above this many particles are ordered by k_fix_big, not by counting
+constexpr int kBigBin = 1024;
+
 struct SortArgs {
-  // particle arrays
-  const int32_t *i1, *i2, *i3;
-  const int16_t *tag;
-  int64_t        npart;
-  int            dim;
-  int            n[3];
-  int            spatial;   // 1: cell key, 0: alive/dead only
-  int            tiled;     // with spatial: tile-major key (tile, then cell in tile)
-  int            tile[3];   // tile shape
-  int            ntiles[3]; // tiles per axis
-  int32_t        dead_bin;  // index of the last bin
+  // particle arrays; the previous positions only when they move too
+  int32_t *i[3], *ip[3];
+  float   *dx[3], *dxp[3];
+  void    *u[4];      // momenta, weight
+  int16_t *tag;
+  int      real_bytes;
+  bool     prev;
+  int64_t  npart;
+  int      dim;
+  int      n[3];
+  int      spatial;   // 1: cell key, 0: alive/dead only
+  int      tiled;     // with spatial: tile-major key (tile, then cell in tile)
+  int      tile_log[3];  // log2 of the tile shape
+  int      ntiles[3]; // tiles per axis
+  int32_t  dead_bin;  // index of the last bin
   // scratch
-  int32_t*  key;
-  int32_t*  rank;
-  uint8_t*  is_dead;
-  int32_t*  dead_rank;
-  int32_t*  count;  // dead_bin + 2 entries
-  int64_t*  off;    // dead_bin + 2 entries
-  int32_t*  perm;
-  int32_t*  perm_tmp;
-  int32_t*  big;
+  int32_t*  rank;     // npart: place of a particle among its bin's, in arrival order
+  int32_t*  dead_off; // one per block of kSortBlock particles: dead before it
+  int32_t*  dead_cnt; // the same, counts
+  int32_t*  count;    // dead_bin + 2 entries
+  int64_t*  off;      // dead_bin + 2 entries
+  int32_t*  perm;     // npart: particle at each place, bins in arrival order (without records)
+  int32_t*  perm2;    // npart: new index -> old index (sort_final_perm)
+  uint4*    rec;      // npart records (null: perm instead)
+  int32_t*  big;      // bins of more than kBigBin particles, at most npart / kBigBin
   int32_t*  nbig;
   unsigned long long* err;
 };
 
-// builds perm (new index -> old index) without host synchronisation; the
-// dead count is left in count[dead_bin]
-cudaError_t sort_build_perm(SortArgs a, cudaStream_t s);
+// 16-byte words of one particle's record (every array above and the index)
+int sort_record_words(int dim, int real_bytes, bool prev);
+
+// counts, offsets and the records (or perm) scattered to their bins, in arrival
+// order within a bin, without host synchronisation. The dead count is left in
+// count[dead_bin]
+cudaError_t sort_scatter(const SortArgs& a, cudaStream_t s);
+// the records back into the particle arrays, each bin in index order
+cudaError_t sort_unpack(const SortArgs& a, cudaStream_t s);
+// the permutation, each bin in index order, into a.perm2; reads the particle
+// arrays' keys, so it comes before sort_unpack
+cudaError_t sort_final_perm(const SortArgs& a, cudaStream_t s);
 
 // every listed array permuted in place: arr_k[i] <- arr_k[perm[i]], staged
 // through tmp_k. With a staging area per array, one kernel gathers all
