@@ -21,6 +21,7 @@
 // cell index is piecewise constant. Shape order >= 2 makes the deposit and
 // interpolation C^1 in X, so the gradient is almost everywhere smooth.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "ctx_internal.cuh"
@@ -212,14 +213,48 @@ struct AdjArgs {
   FieldView<real> lam;   // adjoint of (E, B'), accumulated (ghost-inclusive)
   PushConsts      pc;
   real            dt, dx, ndth, inv_dt, charge;
+  int             lam_count = 0;  // elements of lam's array (row views)
 };
 
+// a 2D field whose x1 neighbours are adjacent and whose elements 32 bits index:
+// the taps of a stencil row are constants away from the row's address
+template <typename real>
+struct RowView {
+  // the rows' additions go as 16-byte vectors (the array starts on 16 bytes)
+  static constexpr bool kVector = sizeof(real) == 4;
+  real*                 p;
+  int                   s1, s3, count;
+  __device__ __forceinline__ RowView(const FieldView<real>& f, int n)
+      : p(f.p), s1((int)f.s1), s3((int)f.s3), count(n) {}
+  // the 16-byte word of this element lies within the array
+  __device__ __forceinline__ bool whole(int i, int j, int c) const {
+    return (j * s1 + c * s3 + i) / 4 * 4 + 4 <= count;
+  }
+  __device__ __forceinline__ real* at(int i, int j, int c) const { return p + (j * s1 + c * s3) + i; }
+  __device__ __forceinline__ real  ld(int i, int j, int, int c) const { return __ldg(at(i, j, c)); }
+};
+template <typename real>
+struct AnyView : FieldView<real> {
+  static constexpr bool kVector = false;
+  __device__ __forceinline__ AnyView(const FieldView<real>& f, int) : FieldView<real>(f) {}
+  __device__ __forceinline__ real* at(int i, int j, int c) const { return this->p + this->idx(i, j, 0, c); }
+};
+
+// V: RowView where the three fields allow it (launch_push_deposit_adjoint):
+// 64-bit addresses with run-time strides were 1,390 of the order-2 kernel's
+// 4,830 instructions per warp. The scatter bounds the kernel at L2: a stencil
+// row's additions go as one or two 16-byte vector reductions instead of O + 1
+// (1.05 M particles, 16 per cell, order 2: 262 -> 247 us with the row views and
+// the shuffle steps cut, 182 with the vectors). Summed in shared-memory windows
+// the field adjoint took 184 us and halved its rounding, but moved the position
+// gradients by 8e-5, more than four times what two runs differ by.
 // FP32 asks for three CTAs per SM (80 registers instead of 128, spilling
 // about 200 bytes): on the two-stream problem the gradient went from 489 to
 // 464 ms, the forward being 128.6 ms
-template <int O, typename real>
+template <int O, typename real, template <typename> class V>
 __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 1)
     k_push_deposit_adjoint(AdjArgs<real> a) {
+  const V<real> EB(a.EB, 0), lamJ(a.lamJ, 0), lam(a.lam, a.lam_count);
   constexpr int N     = O + 2;
   const real    ONE   = 1, HALF = 0.5;
   const real    THIRD = K<real>::THIRD;
@@ -278,7 +313,7 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 1)
           real r = 0, rd = 0;
 #pragma unroll
           for (int ai = 0; ai < O + 1; ai++) {
-            const real F = a.EB.ld(m0 + ai, m1 + bj, 0, c);
+            const real F = EB.ld(m0 + ai, m1 + bj, 0, c);
             r            = iacc(s0 ? Sd[0][ai] : Sp[0][ai], F, r);
             rd += (s0 ? dSd[0][ai] : dSp[0][ai]) * F;
           }
@@ -323,7 +358,7 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 1)
         real       A  = 0;
 #pragma unroll
         for (int i = N - 2; i >= 0; --i) {
-          if (i < d1 && j <= d2) A += a.lamJ.ld(i0s + i, j0s + j, 0, 0);
+          if (i < d1 && j <= d2) A += lamJ.ld(i0s + i, j0s + j, 0, 0);
           const real hd = HALF * (fS[0][i] - iS[0][i]);
           const real tA = -a.inv_dt * A;
           Fu += tA * hd * s1;
@@ -341,7 +376,7 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 1)
         real       A  = 0;
 #pragma unroll
         for (int j = N - 2; j >= 0; --j) {
-          if (i <= d1 && j < d2) A += a.lamJ.ld(i0s + i, j0s + j, 0, 1);
+          if (i <= d1 && j < d2) A += lamJ.ld(i0s + i, j0s + j, 0, 1);
           const real ds = fS[1][j] - iS[1][j];
           const real tA = -a.inv_dt * A;
           Fu += tA * hs * ds;
@@ -367,7 +402,7 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 1)
 #pragma unroll
           for (int j = 0; j < N; ++j) {
             if (!(i <= d1 && j <= d2)) continue;
-            const real l = THIRD * a.lamJ.ld(i0s + i, j0s + j, 0, 2);
+            const real l = THIRD * lamJ.ld(i0s + i, j0s + j, 0, 2);
             F3 += l * (fS[1][j] * ga + iS[1][j] * gb);
             H1f[j] += l * ga;
             H1i[j] += l * gb;
@@ -438,42 +473,74 @@ __global__ void __launch_bounds__(256, sizeof(real) == 4 ? 3 : 1)
     // no shuffles at all when every lane has its own stencil
     const unsigned runlen = head ? (unsigned)(last - lane + 1) : 1u;
     const unsigned maxrun = __reduce_max_sync(0xffffffffu, runlen);
+    // shuffle steps that the longest run needs (a lane's run mates are its
+    // successors; further steps would add nothing)
+    auto scatter = [&](auto steps) {
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      const int s0 = stag_of(c, 0), s1 = stag_of(c, 1);
-      const int m0 = s0 ? dmin[0] : pmin[0];
-      const int m1 = s1 ? dmin[1] : pmin[1];
+      for (int c = 0; c < 6; ++c) {
+        const int s0 = stag_of(c, 0), s1 = stag_of(c, 1);
+        const int m0 = s0 ? dmin[0] : pmin[0];
+        const int m1 = s1 ? dmin[1] : pmin[1];
 #pragma unroll
-      for (int bj = 0; bj < O + 1; bj++) {
+        for (int bj = 0; bj < O + 1; bj++) {
+          real row[O + 1];
 #pragma unroll
-        for (int ai = 0; ai < O + 1; ai++) {
-          real v = lv6[c] * (s0 ? Sd[0][ai] : Sp[0][ai]) * (s1 ? Sd[1][bj] : Sp[1][bj]);
-          if (maxrun > 1) {
+          for (int ai = 0; ai < O + 1; ai++) {
+            real v = lv6[c] * (s0 ? Sd[0][ai] : Sp[0][ai]) * (s1 ? Sd[1][bj] : Sp[1][bj]);
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
+            for (int off = 1; off < (1 << decltype(steps)::value); off <<= 1) {
               const real t = __shfl_down_sync(0xffffffffu, v, off);
               if (lane + off <= last) v += t;
             }
+            row[ai] = v;
           }
-          if (head && valid) atomicAdd(a.lam.p + a.lam.idx(m0 + ai, m1 + bj, 0, c), v);
+          if (head && valid) {
+            if constexpr (V<real>::kVector) {
+              if (lam.whole(m0 + O, m1 + bj, c)) {
+                red_row<O + 1>(lam.at(m0, m1 + bj, c), row);
+                continue;
+              }
+            }
+#pragma unroll
+            for (int ai = 0; ai < O + 1; ai++) atomicAdd(lam.at(m0 + ai, m1 + bj, c), row[ai]);
+          }
         }
       }
-    }
+    };
+    if (maxrun == 1)      scatter(std::integral_constant<int, 0>{});
+    else if (maxrun <= 4) scatter(std::integral_constant<int, 2>{});
+    else if (maxrun <= 8) scatter(std::integral_constant<int, 3>{});
+    else                  scatter(std::integral_constant<int, 5>{});
   }
 }
 
 template <typename real>
-cudaError_t launch_push_deposit_adjoint(int order, const AdjArgs<real>& a, cudaStream_t s) {
-  if (a.sp.npart <= 0) return cudaSuccess;
-  int64_t blocks = (a.sp.npart + 255) / 256;
+cudaError_t launch_push_deposit_adjoint(int order, const AdjArgs<real>& args, cudaStream_t s) {
+  if (args.sp.npart <= 0) return cudaSuccess;
+  int64_t blocks = (args.sp.npart + 255) / 256;
   if (blocks > pic::sm_count() * 32) blocks = pic::sm_count() * 32;
   const unsigned g = (unsigned)blocks;
+  // every element within 32-bit reach of each array's start, x1 packed
+  auto packed = [&](const FieldView<real>& f, int ncomp) {
+    return f.s0 == 1 &&
+           args.pc.ext[0] + (args.pc.ext[1] - 1) * f.s1 + (ncomp - 1) * f.s3 < INT32_MAX - 4;
+  };
+  AdjArgs<real> a = args;
+  const bool    rows = packed(a.EB, 6) && packed(a.lam, 6) && packed(a.lamJ, 3) &&
+                    (uintptr_t)a.lam.p % 16 == 0;
+  if (rows) a.lam_count = (int)(a.pc.ext[0] + (a.pc.ext[1] - 1) * a.lam.s1 + 5 * a.lam.s3);
+#define PIC_ADJ(OO)                                                                            \
+  case OO:                                                                                     \
+    if (rows) PIC_KL(k_push_deposit_adjoint<OO, real, RowView><<<g, 256, 0, s>>>(a));          \
+    else      PIC_KL(k_push_deposit_adjoint<OO, real, AnyView><<<g, 256, 0, s>>>(a));          \
+    break;
   switch (order) {
-    case 1: PIC_KL(k_push_deposit_adjoint<1, real><<<g, 256, 0, s>>>(a)); break;
-    case 2: PIC_KL(k_push_deposit_adjoint<2, real><<<g, 256, 0, s>>>(a)); break;
-    case 3: PIC_KL(k_push_deposit_adjoint<3, real><<<g, 256, 0, s>>>(a)); break;
+    PIC_ADJ(1)
+    PIC_ADJ(2)
+    PIC_ADJ(3)
     default: return cudaErrorInvalidValue;
   }
+#undef PIC_ADJ
   return cudaGetLastError();
 }
 

@@ -217,10 +217,10 @@ constexpr size_t moment_smem() {
 // holds), it sums them in a shared-memory window in fixed point, scaled by the
 // block's largest coefficient, and adds the window's nodes to the grid once;
 // particles apart from the others (across a periodic edge, after a drift) add
-// to the grid directly, and so does a whole block in random order, or one whose
-// coefficients the scale does not suit: not finite, too small, or so unequal
-// (kMomSpread, kMomWeights) that 30 bits below the largest would tell in cells
-// that hold small ones only. FP64 adds to the grid directly: the fixed point
+// to the grid directly, and so does a whole block in random order. Where the
+// block's coefficients do not suit the scale (not finite, too small, or so
+// unequal (kMomSpread, kMomWeights) that 30 bits below the largest would tell
+// in cells that hold small ones only) the window sums in double. FP64 adds to the grid directly: the fixed point
 // would be coarser than double.
 // A particle makes (2 W + 1)^D additions, which bound the kernel. 16.8 M
 // sorted particles at order 2 took 1.64 ms with global atomics, which meet in
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<real> a,
       moment_on_grid<D, ORDER, real>(a, cell, dx, coeff);
       continue;
     }
-    // beyond what the fixed-point scale covers the queue goes onto the grid
+    // beyond what the fixed-point scale covers
     const float m = fabsf((float)coeff);
     bad  = bad || !(m <= 0x1p126f) || (coeff != (real)0 && m < 0x1p-90f);
     cmax = fmaxf(cmax, m);
@@ -369,31 +369,37 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<real> a,
   const int  b     = FA::bits(kMomChunk);
   const real scale = (real)ldexpf(1.f, b - ex), unscale = (real)ldexpf(1.f, ex - b);
   const int  mine  = (int)min(s_cnt[lane], (unsigned)ROWS);
+  double*    sums  = reinterpret_cast<double*>(win);  // two words a node as well
   for (int row = tid >> 5; row < mine; row += kMomThreads / 32) {
     const int e = row * 32 + lane, word = qu.word[e];
     float     dx[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) dx[d] = qu.dx[d][e];
-    if (!fixed) {
-      const int cell[3] = { word % wn[0] + w0[0] + W, word / wn[0] % wn[1] + w0[1] + W,
-                            word / (wn[0] * wn[1]) + w0[2] + W };
-      moment_on_grid<D, ORDER, real>(a, cell, dx, qu.coeff[e]);
-      continue;
-    }
     const MomShape<D, ORDER, real> S(dx, a.smoothing == PIC_SMOOTH_SPLINE);
-    const real                     cs = qu.coeff[e] * scale;
-    S.each([&](int i, int j, int k, real sh) {
-      FA::add(win + word + i + wn[0] * (j + wn[1] * k), nodes, cs * sh);
-    });
+    const real                     coeff = qu.coeff[e], cs = coeff * scale;
+    if (fixed)
+      S.each([&](int i, int j, int k, real sh) {
+        FA::add(win + word + i + wn[0] * (j + wn[1] * k), nodes, cs * sh);
+      });
+    else
+      S.each([&](int i, int j, int k, real sh) {
+        atomicAdd(sums + word + i + wn[0] * (j + wn[1] * k), (double)(coeff * sh));
+      });
   }
-  if (!fixed) return;
   __syncthreads();
   for (int e = tid; e < nodes; e += kMomThreads) {
-    if (!FA::nonzero(win + e, nodes)) continue;
+    real v;
+    if (fixed) {
+      if (!FA::nonzero(win + e, nodes)) continue;
+      v = FA::to_real(FA::total(win + e, nodes), unscale);
+    } else {
+      v = (real)sums[e];
+      if (v == (real)0) continue;
+    }
     const int i = e % wn[0], j = (e / wn[0]) % wn[1], k = e / (wn[0] * wn[1]);
     atomicAdd(a.buf.p + a.buf.idx(w0[0] + i + a.ng, w0[1] + j + a.ng, D == 3 ? w0[2] + k + a.ng : 0,
                                   a.comp),
-              FA::to_real(FA::total(win + e, nodes), unscale));
+              v);
   }
 }
 

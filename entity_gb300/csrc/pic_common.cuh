@@ -608,14 +608,14 @@ __device__ __forceinline__ void deposit_velocity(const Prtl<real>& q, real dx, r
   vp[2] *= inv_energy;
 }
 
-template <int D, int O, typename real, bool FACTORED = false, typename Add>
+template <int D, int O, typename real, bool FACTORED = false, int BOX = BOX_ANY, typename Add>
 __device__ __forceinline__ bool deposit_particle(const Prtl<real>& q, real weight, real charge,
                                                  real inv_dt, real dx, int ng, const int* ext,
                                                  Add&& add) {
   real vp[3];
   deposit_velocity<D, real>(q, dx, vp);
-  return deposit_with_velocity<D, O, real, BOX_ANY, FACTORED>(q, vp, weight, charge, inv_dt, ng,
-                                                              ext, add);
+  return deposit_with_velocity<D, O, real, BOX, FACTORED>(q, vp, weight, charge, inv_dt, ng, ext,
+                                                          add);
 }
 
 // the deposit proper, given the particle velocity vp (the GR deposit passes
@@ -626,7 +626,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
                                                       int ng, const int* ext, Add&& add) {
   constexpr bool UNMOVED = BOX == BOX_UNMOVED;
   static_assert(BOX == BOX_ANY || O >= 1, "the zigzag deposit has no support box");
-  static_assert(FACTORED || BOX == BOX_ANY, "the reference's form takes any extent");
+  static_assert(FACTORED || BOX != BOX_UNMOVED, "the reference's form takes any extent");
   const real ONE = 1, HALF = 0.5, INV_2 = 0.5;
   if constexpr (O == 0) {
     if (ext) {
@@ -714,6 +714,12 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
     constexpr real THIRD = K<real>::THIRD;
     const real     Q     = coeff * inv_dt;
     if constexpr (!FACTORED) {
+      // the add of an entry inside the particle's extent; in a full box an
+      // entry outside adds an exact zero
+      auto put = [&](bool in, int i, int j, int k, int c, real v) {
+        if constexpr (BOX == BOX_FULL) add(i, j, k, c, in ? v : (real)0);
+        else if (in) add(i, j, k, c, v);
+      };
       const int  d1 = imax[0] - imin[0], d2 = imax[1] - imin[1];
       const int  i0 = imin[0] + ng, j0 = imin[1] + ng;
       // Every entry of the (O+2)-wide stencil is computed and only the add is
@@ -737,7 +743,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
           for (int i = 0; i < N - 1; ++i) {
             const real W = hd0[i] * s1;
             acc          = (i == 0) ? (-Q * W) : (acc - Q * W);
-            if (i < d1 && j <= d2) add(i0 + i, j0 + j, 0, 0, acc);
+            put(i < d1 && j <= d2, i0 + i, j0 + j, 0, 0, acc);
           }
         }
         // jx2: prefix over j
@@ -748,7 +754,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
           for (int j = 0; j < N - 1; ++j) {
             const real W = hs0[i] * (fS[1][j] - iS[1][j]);
             acc          = (j == 0) ? (-Q * W) : (acc - Q * W);
-            if (i <= d1 && j < d2) add(i0 + i, j0 + j, 0, 1, acc);
+            put(i <= d1 && j < d2, i0 + i, j0 + j, 0, 1, acc);
           }
         }
         // jx3
@@ -759,7 +765,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
 #pragma unroll
           for (int j = 0; j < N; ++j) {
             const real W = THIRD * (fS[1][j] * ga + iS[1][j] * gb);
-            if (i <= d1 && j <= d2) add(i0 + i, j0 + j, 0, 2, QVx3 * W);
+            put(i <= d1 && j <= d2, i0 + i, j0 + j, 0, 2, QVx3 * W);
           }
         }
       } else {
@@ -785,7 +791,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
             for (int i = 0; i < N - 1; ++i) {
               const real W = t0[i] * P;
               acc          = (i == 0) ? (-Q * W) : (acc - Q * W);
-              if (ok && i < d1) add(i0 + i, j0 + j, k0 + k, 0, acc);
+              put(ok && i < d1, i0 + i, j0 + j, k0 + k, 0, acc);
             }
           }
         }
@@ -802,7 +808,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
             for (int j = 0; j < N - 1; ++j) {
               const real W = t1[j] * P;
               acc          = (j == 0) ? (-Q * W) : (acc - Q * W);
-              if (ok && j < d2) add(i0 + i, j0 + j, k0 + k, 1, acc);
+              put(ok && j < d2, i0 + i, j0 + j, k0 + k, 1, acc);
             }
           }
         }
@@ -819,7 +825,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
             for (int k = 0; k < N - 1; ++k) {
               const real W = t2[k] * P;
               acc          = (k == 0) ? (-Q * W) : (acc - Q * W);
-              if (ok && k < d3) add(i0 + i, j0 + j, k0 + k, 2, acc);
+              put(ok && k < d3, i0 + i, j0 + j, k0 + k, 2, acc);
             }
           }
         }
@@ -915,6 +921,35 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
     }
   }
   return true;
+}
+
+// Adds r[0 .. N - 1] (N <= 4) to N consecutive floats from p on with 16-byte
+// vector reductions: one, or two where they straddle a 16-byte boundary, zeros
+// filling up. The caller vouches for whole 16-byte words around them.
+template <int N>
+__device__ __forceinline__ void red_row(float* p, const float* r) {
+  static_assert(N >= 1 && N <= 4, "at most four floats");
+  const int a = (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3);
+  // the row shifted right by a slots
+  float u[5] = { 0.f, 0.f, 0.f, 0.f, 0.f }, t[8];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const float even = k < N ? r[k < N ? k : 0] : 0.f, odd = k > 0 && k <= N ? r[k > 0 && k <= N ? k - 1 : 0] : 0.f;
+    u[k] = a & 1 ? odd : even;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float lo = k < 5 ? u[k < 5 ? k : 0] : 0.f, hi = k >= 2 && k < 7 ? u[k >= 2 && k < 7 ? k - 2 : 0] : 0.f;
+    t[k] = a & 2 ? hi : lo;
+  }
+  float* q = p - a;
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(q), "f"(t[0]), "f"(t[1]),
+               "f"(t[2]), "f"(t[3])
+               : "memory");
+  if (a + N > 4)
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(q + 4), "f"(t[4]), "f"(t[5]),
+                 "f"(t[6]), "f"(t[7])
+                 : "memory");
 }
 
 // true when the cell of every simulated axis lies in [0, n)
