@@ -211,6 +211,7 @@ __device__ __forceinline__ void for_deposit_unmoved(int i_init, real di_init, in
 // ---------------------------------------------------------------------------
 template <typename real>
 struct FieldView {
+  static constexpr bool kRows = false;
   real*   p;
   int64_t s0, s1, s2, s3;
   __device__ __forceinline__ int64_t idx(int i, int j, int k, int c) const {
@@ -221,10 +222,63 @@ struct FieldView {
   }
 };
 
+// A float field whose x1 neighbours are adjacent, whose array starts on 16 bytes
+// and whose elements 32 bits index: a stencil row is read as one or two 16-byte
+// words. Particles in random order are bound by the lines their reads touch in
+// L1, one per load and lane: a row of O + 1 values then counts 1.25 to 1.75
+// instead of O + 1.
+struct VecField {
+  static constexpr bool kRows = true;
+  const float*          p;
+  int                   s1, s2, s3, count;  // count: elements of the array
+  __device__ __forceinline__ VecField(const FieldView<float>& f, int n)
+      : p(f.p), s1((int)f.s1), s2((int)f.s2), s3((int)f.s3), count(n) {}
+  __device__ __forceinline__ float ld(int i, int j, int k, int c) const {
+    return __ldg(p + (i + j * s1 + k * s2 + c * s3));
+  }
+  // the 16-byte words that hold the rows of N nodes per axis from (i, j, k) on
+  // lie within the array, for every component
+  template <int N>
+  __device__ __forceinline__ bool covers(int i, int j, int k) const {
+    return i + (j + N) * s1 + (k + N) * s2 + 5 * s3 + N + 8 <= count;
+  }
+  // no branch: the loads of a stencil's rows are in flight together
+  template <int N>
+  __device__ __forceinline__ void row(int i, int j, int k, int c, float* r) const {
+    static_assert(N >= 1 && N <= 4, "at most four floats");
+    const int    idx = i + j * s1 + k * s2 + c * s3, a = idx & 3;
+    const float* q = p + (idx - a);
+    const float4 v = __ldg(reinterpret_cast<const float4*>(q));
+    float4       w = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm("{\n\t.reg .pred t;\n\tsetp.gt.s32 t, %4, 4;\n\t"
+        "@t ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%5];\n\t}"
+        : "+f"(w.x), "+f"(w.y), "+f"(w.z), "+f"(w.w)
+        : "r"(a + N), "l"(q + 4));
+    const float x[7] = { v.x, v.y, v.z, v.w, w.x, w.y, w.z };
+    float       t[5];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) t[n] = a & 2 ? x[n + 2] : x[n];
+#pragma unroll
+    for (int n = 0; n < N; ++n) r[n] = a & 1 ? t[n + 1] : t[n];
+  }
+};
+
+// N values along x1 from (i, j, k) on
+template <int N, typename real, typename V>
+__device__ __forceinline__ void load_row(const V& f, int i, int j, int k, int c, real* r) {
+  if constexpr (V::kRows) {
+    f.template row<N>(i, j, k, c, r);
+  } else {
+#pragma unroll
+    for (int n = 0; n < N; ++n) r[n] = f.ld(i + n, j, k, c);
+  }
+}
+
 // a window of a field staged in shared memory: ghost-inclusive index g maps
 // to window index g - off along every axis; 32-bit strides
 template <typename real>
 struct SmemView {
+  static constexpr bool kRows = false;
   const real* p;
   int         off0, off1, off2;
   int         s1, s2, s3;
@@ -337,20 +391,21 @@ __device__ __forceinline__ void unpack(F2 a, float& lo, float& hi) {
 
 // one component's running sums c += S * EB (sr.hpp:1151-1369), products and
 // sums rounded separately; a sum starts with its first product (0 + x is x up
-// to the sign of a zero). T is real, or F2 for two components at once; ld(a,
-// b, c) reads tap (a, b, c), Sx, Sy and Sz are the taps' weights.
-template <int D, int O, typename T, typename Ld, typename WX, typename WY, typename WZ>
-__device__ __forceinline__ T interp_sum(Ld&& ld, WX&& Sx, WY&& Sy, WZ&& Sz) {
+// to the sign of a zero). T is real, or F2 for two components at once; row(b,
+// c, t) reads the taps t[a] of row (b, c), Sx, Sy and Sz are the taps' weights.
+template <int D, int O, typename T, typename Row, typename WX, typename WY, typename WZ>
+__device__ __forceinline__ T interp_sum(Row&& row, WX&& Sx, WY&& Sy, WZ&& Sz) {
   T v;
 #pragma unroll
   for (int c = 0; c < (D == 3 ? O + 1 : 1); ++c) {
     T c0;
 #pragma unroll
     for (int b = 0; b < O + 1; ++b) {
-      T c00;
+      T c00, tap[O + 1];
+      row(b, c, tap);
 #pragma unroll
       for (int a = 0; a < O + 1; ++a) {
-        const T t = Sx(a) * ld(a, b, c);
+        const T t = Sx(a) * tap[a];
         c00       = a == 0 ? t : c00 + t;
       }
       const T t = c00 * Sy(b);
@@ -395,9 +450,12 @@ __device__ __forceinline__ void interp_shape(const V& EB, const int* ic,
         if constexpr (D == 3) Z[k] = f2(S[za][2][k], S[zb][2][k]);
       }
       const F2 r = interp_sum<D, O, F2>(
-        [&](int a, int b, int c) {
-          return f2(EB.ld(mn[xa][0] + a, mn[ya][1] + b, D == 3 ? mn[za][2] + c : 0, ca),
-                    EB.ld(mn[xb][0] + a, mn[yb][1] + b, D == 3 ? mn[zb][2] + c : 0, cb));
+        [&](int b, int c, F2* t) {
+          real u[O + 1], w[O + 1];
+          load_row<O + 1>(EB, mn[xa][0], mn[ya][1] + b, D == 3 ? mn[za][2] + c : 0, ca, u);
+          load_row<O + 1>(EB, mn[xb][0], mn[yb][1] + b, D == 3 ? mn[zb][2] + c : 0, cb, w);
+#pragma unroll
+          for (int a = 0; a < O + 1; ++a) t[a] = f2(u[a], w[a]);
         },
         [&](int k) { return X[k]; }, [&](int k) { return Y[k]; }, [&](int k) { return Z[k]; });
       unpack(r, out[ca], out[cb]);
@@ -407,8 +465,8 @@ __device__ __forceinline__ void interp_shape(const V& EB, const int* ic,
     for (int c = 0; c < 6; ++c) {
       const int x = stag_of(c, 0), y = stag_of(c, 1), z = stag_of(c, 2);
       out[c] = interp_sum<D, O, real>(
-        [&](int a, int b, int k) {
-          return EB.ld(mn[x][0] + a, mn[y][1] + b, D == 3 ? mn[z][2] + k : 0, c);
+        [&](int b, int k, real* t) {
+          load_row<O + 1>(EB, mn[x][0], mn[y][1] + b, D == 3 ? mn[z][2] + k : 0, c, t);
         },
         [&](int k) { return S[x][0][k]; }, [&](int k) { return S[y][1][k]; },
         [&](int k) { return S[z][2][k]; });
@@ -950,6 +1008,110 @@ __device__ __forceinline__ void red_row(float* p, const float* r) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(q + 4), "f"(t[4]), "f"(t[5]),
                  "f"(t[6]), "f"(t[7])
                  : "memory");
+}
+
+// The deposit's reference form (orders 1-3, FP32) by rows along x1:
+// row(n, i, j, k, c, r) adds r[0 .. n - 1] to component c at nodes (i .. i + n - 1,
+// j, k), ghost-inclusive, entries outside the particle's extent being zero.
+// Every entry is deposit_with_velocity's, to the bit. False when the stencil
+// leaves the extents.
+template <int D, int O, typename Row>
+__device__ __forceinline__ bool deposit_rows(const Prtl<float>& q, float vx3, float weight,
+                                             float charge, float inv_dt, int ng, const int* ext,
+                                             Row&& row) {
+  constexpr int N = O + 2;
+  const float   HALF = 0.5f, THIRD = K<float>::THIRD;
+  float         iS[D][N], fS[D][N];
+  int           lo[3] = { 0, 0, 0 }, d[3] = { 0, 0, 0 };
+#pragma unroll
+  for (int a = 0; a < D; ++a) {
+    int hi;
+    for_deposit<O>(q.ip[a], q.dxp[a], q.i[a], q.dx[a], lo[a], hi, iS[a], fS[a]);
+    if (lo[a] + ng < 0 || hi + ng >= ext[a]) return false;
+    d[a] = hi - lo[a];
+    lo[a] += ng;
+  }
+  const float coeff = weight * charge, Q = coeff * inv_dt;
+  auto        next  = [&](int n, float acc, float W) { return n == 0 ? -Q * W : acc - Q * W; };
+  if constexpr (D == 2) {
+    const float QVx3 = coeff * vx3;
+    float       hs0[N], acc[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) hs0[i] = HALF * (fS[0][i] + iS[0][i]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const float s1 = fS[1][j] + iS[1][j], ds = fS[1][j] - iS[1][j];
+      float       r1[N - 1], r2[N], r3[N], a1 = 0;
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (i < N - 1) {
+          a1    = next(i, a1, (HALF * (fS[0][i] - iS[0][i])) * s1);
+          r1[i] = i < d[0] ? a1 : 0.f;
+        }
+        if (j < N - 1) {
+          acc[i] = next(j, acc[i], hs0[i] * ds);
+          r2[i]  = i <= d[0] ? acc[i] : 0.f;
+        }
+        const float ga = HALF * iS[0][i] + fS[0][i], gb = HALF * fS[0][i] + iS[0][i];
+        r3[i]          = i <= d[0] ? QVx3 * (THIRD * (fS[1][j] * ga + iS[1][j] * gb)) : 0.f;
+      }
+      if (j <= d[1]) {
+        row(std::integral_constant<int, N - 1>{}, lo[0], lo[1] + j, 0, 0, r1);
+        row(std::integral_constant<int, N>{}, lo[0], lo[1] + j, 0, 2, r3);
+      }
+      if (j < N - 1 && j < d[1]) row(std::integral_constant<int, N>{}, lo[0], lo[1] + j, 0, 1, r2);
+    }
+  } else {
+    float t[3][N];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int i = 0; i < N; ++i) t[a][i] = THIRD * (fS[a][i] - iS[a][i]);
+    // jx1
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        const float P = (iS[1][j] * iS[2][k] + fS[1][j] * fS[2][k]) +
+                        HALF * (iS[2][k] * fS[1][j] + iS[1][j] * fS[2][k]);
+        float r[N - 1], acc = 0;
+#pragma unroll
+        for (int i = 0; i < N - 1; ++i) {
+          acc  = next(i, acc, t[0][i] * P);
+          r[i] = i < d[0] ? acc : 0.f;
+        }
+        if (j <= d[1] && k <= d[2])
+          row(std::integral_constant<int, N - 1>{}, lo[0], lo[1] + j, lo[2] + k, 0, r);
+      }
+    // jx2, prefix along x2, and jx3, along x3: a = the moving axis, b the other
+#pragma unroll
+    for (int a = 1; a < 3; ++a) {
+      const int b = 3 - a;
+#pragma unroll
+      for (int m = 0; m < N; ++m) {  // along b
+        float P[N], acc[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+          P[i] = a == 1 ? iS[0][i] * iS[b][m] + fS[0][i] * fS[b][m] +
+                            HALF * (iS[b][m] * fS[0][i] + iS[0][i] * fS[b][m])
+                        : iS[0][i] * iS[b][m] + fS[0][i] * fS[b][m] +
+                            HALF * (iS[0][i] * fS[b][m] + iS[b][m] * fS[0][i]);
+#pragma unroll
+        for (int l = 0; l < N - 1; ++l) {  // along a
+          float r[N];
+#pragma unroll
+          for (int i = 0; i < N; ++i) {
+            acc[i] = next(l, acc[i], t[a][l] * P[i]);
+            r[i]   = i <= d[0] ? acc[i] : 0.f;
+          }
+          if (l < d[a] && m <= d[b])
+            row(std::integral_constant<int, N>{}, lo[0], lo[1] + (a == 1 ? l : m),
+                lo[2] + (a == 1 ? m : l), a, r);
+        }
+      }
+    }
+  }
+  return true;
 }
 
 // true when the cell of every simulated axis lies in [0, n)
