@@ -283,11 +283,12 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
   PIC_TD(3, 3)
 #undef PIC_TD
   if (e != cudaSuccess) return PIC_ERR_CUDA;
-  // the particles the tiled kernel deferred: per-particle kernel over the list
+  // the particles the tiled kernel deferred: per-particle kernel over the lists
+  pic::DrainArgs<real> dr;
+  dr.n = a.nsp;
   for (int k = 0; k < a.nsp; ++k) {
-    const pic_species* sp = sps[k];
-    pic::PDArgs<real>  pa;
-    pa.sp = sptrs(sp);
+    pic::PDArgs<real>& pa = dr.s[k];
+    pa.sp = sptrs(sps[k]);
     pa.pc = a.pc;
     pa.EB = a.EB;
     pa.J  = a.J;
@@ -302,10 +303,20 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
     pa.list       = a.s[k].ovf;
     pa.list_count = a.s[k].ovf_count;
     pa.fj         = a.fj;
-    e = pd_dispatch<real>(c, pa, pic::MODE_FUSED, false, s);
-    if (e != cudaSuccess) return PIC_ERR_CUDA;
   }
-  return PIC_OK;
+  e = cudaErrorInvalidValue;
+#define PIC_DR(DD, OO) \
+  if (D == DD && O == OO) e = pic::launch_push_deposit_lists<DD, OO, real>(dr, s);
+  PIC_DR(2, 0)
+  PIC_DR(2, 1)
+  PIC_DR(2, 2)
+  PIC_DR(2, 3)
+  PIC_DR(3, 0)
+  PIC_DR(3, 1)
+  PIC_DR(3, 2)
+  PIC_DR(3, 3)
+#undef PIC_DR
+  return cuda_status(e);
 }
 
 template <typename real>

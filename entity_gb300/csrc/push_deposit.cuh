@@ -134,8 +134,7 @@ __device__ __forceinline__ void fixed_scale(const FixedJ& fj, float& scale, int&
 // order 2 pushed in 5.43 and deposited in 3.92 ms without, 4.11 and 2.25 with
 // (three blocks per SM for the deposit: 2.22, two 2.38, one 2.76 ms).
 template <int D, int O, typename real, int MODE, bool PHOTON, bool VEC>
-__global__ void __launch_bounds__(256, (D == 2 && sizeof(real) == 4) ? 3 : (VEC ? (MODE == MODE_DEPOSIT ? 3 : 2) : 1))
-    k_push_deposit(PDArgs<real> a) {
+__device__ __forceinline__ void push_deposit_all(const PDArgs<real>& a) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t n = a.list ? (int64_t)*a.list_count : a.sp.npart;
   // exact accumulator: each contribution is rounded to a multiple of
@@ -211,6 +210,31 @@ __global__ void __launch_bounds__(256, (D == 2 && sizeof(real) == 4) ? 3 : (VEC 
       if (!ok) atomicAdd(a.err + ERR_STENCIL_OUT, 1ull);
     }
   }
+}
+
+template <int D, int O, typename real, int MODE, bool PHOTON, bool VEC>
+__global__ void __launch_bounds__(256, (D == 2 && sizeof(real) == 4)
+                                           ? 3
+                                           : (VEC ? (MODE == MODE_DEPOSIT ? 3 : 2) : 1))
+    k_push_deposit(const __grid_constant__ PDArgs<real> a) {
+  push_deposit_all<D, O, real, MODE, PHOTON, VEC>(a);
+}
+
+// The particles that a tiled launch left to this kernel, every species' list in
+// one launch (blockIdx.y). The lists are short and a particle is one long chain
+// of latencies, so the lists share the SMs: two of 512^2 pairs took 9.5 us each
+// in launches of their own, 14 us together, two of 100 x 75 x 61 turbulence 25
+// and 45 us.
+constexpr int kMaxTiledSpecies = 4;
+template <typename real>
+struct DrainArgs {
+  PDArgs<real> s[kMaxTiledSpecies];
+  int          n = 0;
+};
+template <int D, int O, typename real>
+__global__ void __launch_bounds__(128, (D == 2 && sizeof(real) == 4) ? 6 : 4)
+    k_push_deposit_lists(const __grid_constant__ DrainArgs<real> d) {
+  push_deposit_all<D, O, real, MODE_FUSED, false, false>(d.s[blockIdx.y]);
 }
 
 // The grid nodes around the cells of a block's n consecutive particles from p0
@@ -343,5 +367,7 @@ __global__ void __launch_bounds__(256, O == 3 ? 3 : 4) k_push_deposit_chunk(cons
 // host-side launcher, explicitly instantiated per (D, O, real)
 template <int D, int O, typename real>
 cudaError_t launch_push_deposit(const PDArgs<real>& a, int mode, bool photon, cudaStream_t s);
+template <int D, int O, typename real>
+cudaError_t launch_push_deposit_lists(const DrainArgs<real>& d, cudaStream_t s);
 
 }  // namespace pic

@@ -51,7 +51,6 @@
 
 namespace pic {
 
-constexpr int kMaxTiledSpecies = 4;
 constexpr int kDriftMargin     = 1;
 
 // tile shape per (dimension, precision, order): the shared-memory windows
