@@ -20,6 +20,7 @@
 #include "ctx_internal.cuh"
 #include "fields.cuh"
 #include "gr_host.cuh"
+#include "gr_island.cuh"
 #include "gr_metric.cuh"
 #include "pic_common.cuh"
 
@@ -35,6 +36,7 @@ struct GRPushArgs {
   SpeciesPtrs     sp;
   FieldView<real> em, em0;
   QKS<double>     m;
+  island::Rcp     rcp;
   int             n1, n2, ng;
   int             absorb_min, absorb_max, axis_min, axis_max;
   real            dt, ndth;
@@ -106,13 +108,42 @@ __device__ __forceinline__ M gamma_of(bool massive, const M* uc, const M* uu) {
   return massive ? sqrt((M)1 + s) : sqrt(s);
 }
 
+__device__ __forceinline__ bool same_bits(float a, float b) {
+  return __float_as_int(a) == __float_as_int(b);
+}
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
+// niter passes of x = f(x) over two components. A pass is a function of x's
+// bits alone, so once it returns its argument, or the argument of the pass
+// before (rounding often leaves x alternating between two neighbours), the
+// passes left are known: the result is the last pass's, bit for bit. The time
+// step is a fraction of the smallest cell, so most particles settle within
+// three of the reference's ten passes.
+template <typename M, typename F>
+__device__ __forceinline__ void iterate2(int niter, M* x, F&& f) {
+  M prev[2] = { x[0], x[1] };
+  for (int it = 0; it < niter; ++it) {
+    M y[2];
+    f(it, x, y);
+    const bool fixed = same_bits(y[0], x[0]) && same_bits(y[1], x[1]);
+    const bool cycle = it > 0 && same_bits(y[0], prev[0]) && same_bits(y[1], prev[1]);
+    if (fixed || (cycle && ((niter - it) & 1))) {
+      x[0] = y[0], x[1] = y[1];
+      return;
+    }
+    if (cycle) return;
+    prev[0] = x[0], prev[1] = x[1];
+    x[0] = y[0], x[1] = y[1];
+  }
+}
+
 // GeodesicMomentumPush (gr.hpp:260-331): the metric and its derivatives at
 // the (fixed) position are formed once for all iterations
 template <typename M>
-__device__ __forceinline__ void geo_momentum(const QKS<M>& m, bool massive, M dt, int niter,
-                                             const M* xp, const M* vp, M* vu) {
-  const QPt<M>  p  = qpt(m, xp[0], xp[1]);
-  const QMet<M> g  = qmet(m, p);
+__device__ __forceinline__ void geo_momentum(const QKS<M>& m, const QPt<M>& p, const QMet<M>& g,
+                                             bool massive, M dt, int niter, const M* vp, M* vu) {
   const M d_al[2] = { dr_alpha(m, p), dt_alpha(m, p) };
   const M d_be[2] = { dr_beta1(m, p), dt_beta1(m, p) };
   const M d_11[2] = { dr_h11(m, p), dt_h11(m, p) };
@@ -120,37 +151,40 @@ __device__ __forceinline__ void geo_momentum(const QKS<M>& m, bool massive, M dt
   const M d_33[2] = { dr_h33(m, p), dt_h33(m, p) };
   const M d_13[2] = { dr_h13(m, p), dt_h13(m, p) };
   vu[0] = vp[0], vu[1] = vp[1], vu[2] = vp[2];
-  for (int it = 0; it < niter; ++it) {
-    const M vm[3] = { (M)0.5 * (vp[0] + vu[0]), (M)0.5 * (vp[1] + vu[1]), vp[2] };
+  iterate2(niter, vu, [&](int, const M* v, M* o) {
+    const M vm[3] = { (M)0.5 * (vp[0] + v[0]), (M)0.5 * (vp[1] + v[1]), vp[2] };
     M       vmc[3];
     d_to_u(g, vm, vmc);
     const M u0 = gamma_of(massive, vm, vmc) / g.alpha;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      vu[k] = vp[k] + dt * (-g.alpha * u0 * d_al[k] + vm[0] * d_be[k] -
-                            ((M)0.5 / u0) *
-                              (d_11[k] * (vm[0] * vm[0]) + d_22[k] * (vm[1] * vm[1]) +
-                               d_33[k] * (vm[2] * vm[2]) + (M)2 * d_13[k] * vm[0] * vm[2]));
+      o[k] = vp[k] + dt * (-g.alpha * u0 * d_al[k] + vm[0] * d_be[k] -
+                           ((M)0.5 / u0) *
+                             (d_11[k] * (vm[0] * vm[0]) + d_22[k] * (vm[1] * vm[1]) +
+                              d_33[k] * (vm[2] * vm[2]) + (M)2 * d_13[k] * vm[0] * vm[2]));
     }
-  }
+  });
 }
 
-// GeodesicCoordinatePush (gr.hpp:333-383)
+// GeodesicCoordinatePush (gr.hpp:333-383); g0 is the metric at (xp[0],
+// clamp_x2(xp[1])), the first pass's midpoint
 template <typename M>
-__device__ __forceinline__ void geo_coordinate(const QKS<M>& m, bool massive, M dt, int niter,
-                                               const M* xp, const M* vp, M* xu) {
+__device__ __forceinline__ void geo_coordinate(const QKS<M>& m, const QMet<M>& g0, bool massive,
+                                               M dt, int niter, const M* xp, const M* vp, M* xu) {
   xu[0] = xp[0], xu[1] = xp[1];
-  for (int it = 0; it < niter; ++it) {
-    const M       xm0 = (M)0.5 * (xp[0] + xu[0]);
-    const M       xm1 = m.clamp_x2((M)0.5 * (xp[1] + xu[1]));
-    const QPt<M>  p   = qpt(m, xm0, xm1);
-    const QMet<M> g   = qmet(m, p);
-    M             vc[3];
+  iterate2(niter, xu, [&](int it, const M* x, M* o) {
+    QMet<M> g = g0;
+    if (it > 0) {
+      const M xm0 = (M)0.5 * (xp[0] + x[0]);
+      const M xm1 = m.clamp_x2((M)0.5 * (xp[1] + x[1]));
+      g           = qmet(m, qpt(m, xm0, xm1));
+    }
+    M vc[3];
     d_to_u(g, vp, vc);
     const M u0 = gamma_of(massive, vp, vc) / g.alpha;
-    xu[0] = xp[0] + dt * (vc[0] / u0 - g.beta1);
-    xu[1] = xp[1] + dt * (vc[1] / u0);
-  }
+    o[0]       = xp[0] + dt * (vc[0] / u0 - g.beta1);
+    o[1]       = xp[1] + dt * (vc[1] / u0);
+  });
 }
 
 template <typename M>
@@ -158,22 +192,25 @@ __device__ __forceinline__ void gr_push_one(const QKS<M>& m, bool massive, M ndt
                                             const M* xp, const M* Dc, const M* Bc, const M* u,
                                             M* xo, M* uo) {
   M vp[3] = { u[0], u[1], u[2] }, vu[3];
+  const M xc = m.clamp_x2(xp[1]);
+  QPt<M>  p  = qpt(m, xp[0], xp[1]);
+  QMet<M> g  = qmet(m, p);
   if (massive) {
-    const M       xq[2] = { xp[0], m.clamp_x2(xp[1]) };
-    const QMet<M> g     = qmet(m, qpt(m, xp[0], xp[1]));
-    M             Dh[3], Bh[3];
+    M Dh[3], Bh[3];
     u_to_t(g, Dc, Dh);
     u_to_t(g, Bc, Bh);
-    em_half_push(g, ndth, vp, Dh, Bh, vu);
+    const QMet<M> ge = g;  // the half pushes' metric is the unclamped point's
+    em_half_push(ge, ndth, vp, Dh, Bh, vu);
     vp[0] = vu[0], vp[1] = vu[1], vp[2] = vu[2];
-    geo_momentum(m, true, dt, niter, xq, vp, vu);
+    if (xc != xp[1]) p = qpt(m, xp[0], xc), g = qmet(m, p);
+    geo_momentum(m, p, g, true, dt, niter, vp, vu);
     vp[0] = vu[0], vp[1] = vu[1], vp[2] = vu[2];
-    em_half_push(g, ndth, vp, Dh, Bh, vu);
-    geo_coordinate(m, true, dt, niter, xp, vu, xo);
+    em_half_push(ge, ndth, vp, Dh, Bh, vu);
   } else {
-    geo_momentum(m, false, dt, niter, xp, vp, vu);
-    geo_coordinate(m, false, dt, niter, xp, vu, xo);
+    geo_momentum(m, p, g, false, dt, niter, vp, vu);
+    if (xc != xp[1]) g = qmet(m, qpt(m, xp[0], xc));
   }
+  geo_coordinate(m, g, massive, dt, niter, xp, vu, xo);
   uo[0] = vu[0], uo[1] = vu[1], uo[2] = vu[2];
 }
 
@@ -207,8 +244,8 @@ __device__ __forceinline__ void gr_push_particle(const GRPushArgs<real>& a, int6
     const double Bd[3] = { (double)Bc[0], (double)Bc[1], (double)Bc[2] };
     const double ud[3] = { (double)ux[0][p], (double)ux[1][p], (double)ux[2][p] };
     double       xd[2], uo_d[3];
-    gr_push_one<double>(a.m, a.massive, (double)a.ndth, (double)a.dt, a.niter, xp, Dd, Bd, ud, xd,
-                        uo_d);
+    island::push_one(a.m, a.rcp, a.massive, (double)a.ndth, (double)a.dt, a.niter, xp, Dd, Bd, ud, xd, uo_d,
+                     [](int n, double* x, auto&& f) { iterate2(n, x, f); });
     xo[0] = (real)xd[0], xo[1] = (real)xd[1];
     uo[0] = (real)uo_d[0], uo[1] = (real)uo_d[1], uo[2] = (real)uo_d[2];
   } else {
@@ -278,8 +315,9 @@ __global__ void __launch_bounds__(256) k_gr_island_list(GRPushArgs<real> a) {
 // precision. With a.list null (FP64 fields, or no island) every particle is
 // pushed here. It asks for three CTAs per SM (80 registers instead of the
 // allocator's 120, a 12-byte spill at order 2): the Wald problem's
-// push+deposit went from 0.718 to 0.608 ms per step; the island kernel at
-// four CTAs of 128 spilled and lost.
+// push+deposit went from 0.718 to 0.608 ms per step. Issue-bound on the
+// metric's divisions: 0.91 million particles took 234 us beside the island
+// with all ten passes, 120 us (87 alone) with passes ended at a fixed point.
 template <int O, typename real>
 __global__ void __launch_bounds__(256, 3) k_gr_push(GRPushArgs<real> a) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -300,9 +338,13 @@ __global__ void __launch_bounds__(256, 3) k_gr_push(GRPushArgs<real> a) {
 // particle arrays; pushed in place, their FP64 work (GB300 runs FP64 at
 // 1/64 of the FP32 rate) would sit on the few SMs holding those blocks. This
 // kernel runs on a second stream beside the bulk, so the FP64 and FP32 pipes
-// work at once.
+// work at once; in blocks of one warp, whose registers are free for the bulk
+// as soon as the list is exhausted. 14 thousand island particles of 0.91
+// million (1024 x 512 Wald problem, order 2): 342 us with the component
+// formulas and all ten passes of both iterations, 235 with passes ended at a
+// fixed point, 133 with island::push_one.
 template <int O, typename real>
-__global__ void __launch_bounds__(128, 3) k_gr_push_island(GRPushArgs<real> a) {
+__global__ void __launch_bounds__(32, 12) k_gr_push_island(GRPushArgs<real> a) {
   const int      lane = threadIdx.x & 31;
   const unsigned n    = a.list_count[0];
   for (;;) {
@@ -899,6 +941,7 @@ pic::GRPushArgs<real> push_args(pic_ctx* c, const pic_gr_metric* g, const pic_sp
   const float qm = sp->pusher == PIC_PUSHER_PHOTON ? 0.0f : sp->charge / sp->mass;
   a.ndth       = (real)0.5 * (real)qm * (real)omegaB0 * (real)dt;
   a.niter      = niter;
+  a.rcp        = { 1.0 / a.m.dchi, 1.0 / a.m.deta };
   a.island_lo  = island_lo;
   a.island_hi  = island_hi;
   a.massive    = sp->pusher != PIC_PUSHER_PHOTON;
@@ -961,12 +1004,12 @@ int gr_push_species(pic_ctx* c, const pic_gr_metric* g, const pic_species* const
     cudaStream_t s2 = c->gr_side[k];
     if (cudaStreamWaitEvent(s2, c->gr_fork, 0) != cudaSuccess) return PIC_ERR_CUDA;
     if constexpr (sizeof(real) == 4) {
-      // three 128-thread blocks per SM fit at up to 170 registers per thread
-      const unsigned bi = (unsigned)pic::sm_count() * 3;
+      // twelve one-warp blocks per SM fit at up to 170 registers per thread
+      const unsigned bi = (unsigned)pic::sm_count() * 12;
       switch (c->grid.order) {
-        case 1: PIC_KL(pic::k_gr_push_island<1, real><<<bi, 128, 0, s2>>>(a[k])); break;
-        case 2: PIC_KL(pic::k_gr_push_island<2, real><<<bi, 128, 0, s2>>>(a[k])); break;
-        default: PIC_KL(pic::k_gr_push_island<3, real><<<bi, 128, 0, s2>>>(a[k])); break;
+        case 1: PIC_KL(pic::k_gr_push_island<1, real><<<bi, 32, 0, s2>>>(a[k])); break;
+        case 2: PIC_KL(pic::k_gr_push_island<2, real><<<bi, 32, 0, s2>>>(a[k])); break;
+        default: PIC_KL(pic::k_gr_push_island<3, real><<<bi, 32, 0, s2>>>(a[k])); break;
       }
     }
     if (cudaEventRecord(c->gr_join[k], s2) != cudaSuccess) return PIC_ERR_CUDA;
