@@ -426,28 +426,55 @@ struct Range2 {
     const int i1 = (R).i0 + (int)(t_ % ((R).i1 - (R).i0));                                 \
     const int i2 = (R).j0 + (int)(t_ / ((R).i1 - (R).i0));
 
+// Rows of R over warps: a warp takes up to kRowChunks spans of W cells of one
+// row, so that the row's part of the metric (the sine and cosine of its two
+// thetas) is formed once per warp; two spans leave enough warps (1024 x 512
+// cells, k_gr_aux_e: 16.6 us with one, 16.1 with two, 18.8 with four). f(i1, lane): every lane of the warp calls it,
+// i1 may lie outside R.
+constexpr int kRowChunks = 2;
+template <int W, typename F, typename S>
+__device__ __forceinline__ void row_spans(const Range2& R, S&& row_start, F&& f) {
+  const int     lane = threadIdx.x & 31, w = R.i1 - R.i0;
+  const int     spans = (w + W - 1) / W, groups = (spans + kRowChunks - 1) / kRowChunks;
+  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int     row = (int)(warp / groups), first = (int)(warp - (int64_t)row * groups) * kRowChunks;
+  if (row >= R.j1 - R.j0) return;
+  row_start(R.j0 + row);
+  for (int k = first; k < min(first + kRowChunks, spans); ++k) f(R.i0 + k * W - (32 - W) / 2 + lane, lane);
+}
+
 template <typename real>
 struct GRFld {
   QKS<double>     m;
   int             ng, n1, n2, axis_min, axis_max;
 };
 
-// Faraday_kernel (faraday_gr.hpp:62-90): Bout = Bin + coeff curl E
+// Faraday_kernel (faraday_gr.hpp:62-90): Bout = Bin + coeff curl E. Bound by
+// the metric's divisions and roots, like the four kernels below; 1024 x 512
+// cells: 12.7 us with every cell's own sines and cosines, 11.5 us.
 template <typename real>
-__global__ void k_gr_faraday(GRFld<real> f, Range2 R, FieldView<real> Bin, FieldView<real> Bout,
-                             FieldView<real> E, real coeff) {
+__global__ void __launch_bounds__(128) k_gr_faraday(GRFld<real> f, Range2 R, FieldView<real> Bin,
+                                                    FieldView<real> Bout, FieldView<real> E,
+                                                    real coeff) {
   const QKS<real> m = f.m.template as<real>();
   const real      H = 0.5;
-  GR_CELL_LOOP(R)
-    const real i1_ = (real)(i1 - f.ng), i2_ = (real)(i2 - f.ng);
-    const real inv_0pH  = (real)1 / sqrt_det_h(m, qpt(m, i1_, i2_ + H));
-    const real inv_pHpH = (real)1 / sqrt_det_h(m, qpt(m, i1_ + H, i2_ + H));
+  int             i2 = 0;
+  QRow<real>      r0, rH;
+  row_spans<32>(R, [&](int j) {
+    i2 = j;
+    r0 = qrow(m, (real)(i2 - f.ng)), rH = qrow(m, (real)(i2 - f.ng) + H);
+  }, [&](int i1, int) {
+    if (i1 >= R.i1) return;
+    const real       i1_ = (real)(i1 - f.ng);
+    const QCol<real> c0 = qcol(m, i1_), cH = qcol(m, i1_ + H);
+    const real inv_0pH  = (real)1 / sqrt_det_h(m, qpt(m, c0, rH));
+    const real inv_pHpH = (real)1 / sqrt_det_h(m, qpt(m, cH, rH));
     Bout.p[Bout.idx(i1, i2, 0, 3)] = Bin.p[Bin.idx(i1, i2, 0, 3)] +
                                      coeff * inv_0pH * (E.p[E.idx(i1, i2, 0, 2)] - E.p[E.idx(i1, i2 + 1, 0, 2)]);
     if (i2 == f.ng && f.axis_min) {
       Bout.p[Bout.idx(i1, i2, 0, 4)] = (real)0;
     } else {
-      const real inv_pH0 = (real)1 / sqrt_det_h(m, qpt(m, i1_ + H, i2_));
+      const real inv_pH0 = (real)1 / sqrt_det_h(m, qpt(m, cH, r0));
       Bout.p[Bout.idx(i1, i2, 0, 4)] =
         Bin.p[Bin.idx(i1, i2, 0, 4)] +
         coeff * inv_pH0 * (E.p[E.idx(i1 + 1, i2, 0, 2)] - E.p[E.idx(i1, i2, 0, 2)]);
@@ -457,28 +484,37 @@ __global__ void k_gr_faraday(GRFld<real> f, Range2 R, FieldView<real> Bin, Field
       coeff * inv_pHpH *
         (E.p[E.idx(i1, i2 + 1, 0, 0)] - E.p[E.idx(i1, i2, 0, 0)] + E.p[E.idx(i1, i2, 0, 1)] -
          E.p[E.idx(i1 + 1, i2, 0, 1)]);
-  }
+  });
 }
 
-// Ampere_kernel (ampere_gr.hpp:66-98) except the axis copies of dx1
+// Ampere_kernel (ampere_gr.hpp:66-98) except the axis copies of dx1 (13.6
+// and 11.2 us)
 template <typename real>
-__global__ void k_gr_ampere(GRFld<real> f, Range2 R, FieldView<real> Din, FieldView<real> Dout,
-                            FieldView<real> Hf, real coeff) {
+__global__ void __launch_bounds__(128) k_gr_ampere(GRFld<real> f, Range2 R, FieldView<real> Din,
+                                                   FieldView<real> Dout, FieldView<real> Hf,
+                                                   real coeff) {
   const QKS<real> m = f.m.template as<real>();
   const real      H = 0.5;
   const int       i2min = f.ng, i2max = f.n2 + f.ng;
-  GR_CELL_LOOP(R)
-    const real i1_ = (real)(i1 - f.ng), i2_ = (real)(i2 - f.ng);
+  int             i2 = 0;
+  QRow<real>      r0, rH;
+  row_spans<32>(R, [&](int j) {
+    i2 = j;
+    r0 = qrow(m, (real)(i2 - f.ng)), rH = qrow(m, (real)(i2 - f.ng) + H);
+  }, [&](int i1, int) {
+    if (i1 >= R.i1) return;
+    const real       i1_ = (real)(i1 - f.ng);
+    const QCol<real> c0 = qcol(m, i1_);
 #define HH(a, b, c) Hf.p[Hf.idx(a, b, 0, c)]
     if (i2 == i2min && f.axis_min) {
-      const real inv = (real)1 / sqrt_det_h(m, qpt(m, i1_, H));
+      const real inv = (real)1 / sqrt_det_h(m, qpt(m, c0, rH));
       Dout.p[Dout.idx(i1, i2, 0, 1)] = Din.p[Din.idx(i1, i2, 0, 1)] +
                                        coeff * inv * (HH(i1 - 1, i2, 5) - HH(i1, i2, 5));
     } else if (i2 == i2max && f.axis_max) {
     } else {
-      const real inv_0pH = (real)1 / sqrt_det_h(m, qpt(m, i1_, i2_ + H));
-      const real inv_00  = (real)1 / sqrt_det_h(m, qpt(m, i1_, i2_));
-      const real inv_pH0 = (real)1 / sqrt_det_h(m, qpt(m, i1_ + H, i2_));
+      const real inv_0pH = (real)1 / sqrt_det_h(m, qpt(m, c0, rH));
+      const real inv_00  = (real)1 / sqrt_det_h(m, qpt(m, c0, r0));
+      const real inv_pH0 = (real)1 / sqrt_det_h(m, qpt(m, qcol(m, i1_ + H), r0));
       Dout.p[Dout.idx(i1, i2, 0, 0)] = Din.p[Din.idx(i1, i2, 0, 0)] +
                                        coeff * inv_pH0 * (HH(i1, i2, 5) - HH(i1, i2 - 1, 5));
       Dout.p[Dout.idx(i1, i2, 0, 1)] = Din.p[Din.idx(i1, i2, 0, 1)] +
@@ -488,7 +524,7 @@ __global__ void k_gr_ampere(GRFld<real> f, Range2 R, FieldView<real> Din, FieldV
         coeff * inv_00 * ((HH(i1, i2 - 1, 3) - HH(i1, i2, 3)) + (HH(i1, i2, 4) - HH(i1 - 1, i2, 4)));
     }
 #undef HH
-  }
+  });
 }
 
 // the axis cells' dx1 = the neighbouring row's (read after that row's update)
@@ -504,103 +540,122 @@ __global__ void k_gr_ampere_axis(GRFld<real> f, FieldView<real> Din, FieldView<r
     Dout.p[Dout.idx(i1, f.n2 + f.ng, 0, 0)] = src.p[src.idx(i1, f.n2 + f.ng - 1, 0, 0)];
 }
 
-// CurrentsAmpere_kernel (ampere_gr.hpp:143-172)
+// CurrentsAmpere_kernel (ampere_gr.hpp:143-172; 11.6 and 10.4 us)
 template <typename real>
-__global__ void k_gr_currents_ampere(GRFld<real> f, Range2 R, FieldView<real> D,
-                                     FieldView<real> J, real coeff) {
+__global__ void __launch_bounds__(128) k_gr_currents_ampere(GRFld<real> f, Range2 R,
+                                                            FieldView<real> D, FieldView<real> J,
+                                                            real coeff) {
   const QKS<real> m = f.m.template as<real>();
   const real      H = 0.5;
   const int       i2min = f.ng, i2max = f.n2 + f.ng;
-  GR_CELL_LOOP(R)
-    const real i1_ = (real)(i1 - f.ng), i2_ = (real)(i2 - f.ng);
-    const real inv_0pH = (real)1 / sqrt_det_h(m, qpt(m, i1_, i2_ + H));
+  int             i2 = 0;
+  QRow<real>      r0, rH;
+  row_spans<32>(R, [&](int j) {
+    i2 = j;
+    r0 = qrow(m, (real)(i2 - f.ng)), rH = qrow(m, (real)(i2 - f.ng) + H);
+  }, [&](int i1, int) {
+    if (i1 >= R.i1) return;
+    const real       i1_ = (real)(i1 - f.ng);
+    const QCol<real> c0 = qcol(m, i1_);
+    const real inv_0pH = (real)1 / sqrt_det_h(m, qpt(m, c0, rH));
     if (i2 == i2min && f.axis_min) {
       D.p[D.idx(i1, i2, 0, 0)] += J.p[J.idx(i1, i2, 0, 0)] * H * coeff / polar_area(m, i1_ + H);
       D.p[D.idx(i1, i2, 0, 1)] += J.p[J.idx(i1, i2, 0, 1)] * coeff * inv_0pH;
     } else if (i2 == i2max && f.axis_max) {
       D.p[D.idx(i1, i2, 0, 0)] += J.p[J.idx(i1, i2, 0, 0)] * H * coeff / polar_area(m, i1_ + H);
     } else {
-      const real inv_00  = (real)1 / sqrt_det_h(m, qpt(m, i1_, i2_));
-      const real inv_pH0 = (real)1 / sqrt_det_h(m, qpt(m, i1_ + H, i2_));
+      const real inv_00  = (real)1 / sqrt_det_h(m, qpt(m, c0, r0));
+      const real inv_pH0 = (real)1 / sqrt_det_h(m, qpt(m, qcol(m, i1_ + H), r0));
       D.p[D.idx(i1, i2, 0, 0)] += J.p[J.idx(i1, i2, 0, 0)] * coeff * inv_pH0;
       D.p[D.idx(i1, i2, 0, 1)] += J.p[J.idx(i1, i2, 0, 1)] * coeff * inv_0pH;
       D.p[D.idx(i1, i2, 0, 2)] += J.p[J.idx(i1, i2, 0, 2)] * coeff * inv_00;
     }
-  }
+  });
 }
 
-// ComputeAuxE_kernel (aux_fields_gr.hpp:47-109)
+// ComputeAuxE_kernel (aux_fields_gr.hpp:47-109). Each cell forms its own four
+// points and the terms of the averages there; the terms of the cells beside
+// it come from the neighbouring lanes (30 cells per warp, one lane more on
+// either side). 1024 x 512 cells: 26 us with seven points per cell, 16 us.
 template <typename real>
-__global__ void k_gr_aux_e(GRFld<real> f, Range2 R, FieldView<real> Df, FieldView<real> Bf,
-                           FieldView<real> Ef) {
+__global__ void __launch_bounds__(128) k_gr_aux_e(GRFld<real> f, Range2 R, FieldView<real> Df,
+                                                  FieldView<real> Bf, FieldView<real> Ef) {
   const QKS<real> m = f.m.template as<real>();
   const real      H = 0.5;
-  GR_CELL_LOOP(R)
-    const real i1_ = (real)(i1 - f.ng), i2_ = (real)(i2 - f.ng);
-#define DD(a, b, c) Df.p[Df.idx(a, b, 0, c)]
-#define BB(a, b, c) Bf.p[Bf.idx(a, b, 0, c)]
-    const QPt<real> p_pH0 = qpt(m, i1_ + H, i2_), p_0pH = qpt(m, i1_, i2_ + H);
-    const QPt<real> p_00 = qpt(m, i1_, i2_), p_mH0 = qpt(m, i1_ - H, i2_);
-    const QPt<real> p_mHpH = qpt(m, i1_ - H, i2_ + H), p_pHpH = qpt(m, i1_ + H, i2_ + H);
-    const QPt<real> p_10 = qpt(m, i1_ + (real)1, i2_);
-    real w1 = sqrt_det_h_tilde(m, p_mH0), w2 = sqrt_det_h_tilde(m, p_pH0);
-    real ww = (real)2 * sqrt_det_h_tilde(m, p_00);
-    const real D1_half = (w1 * h_13(m, p_mH0) * DD(i1 - 1, i2, 0) + w2 * h_13(m, p_pH0) * DD(i1, i2, 0)) / ww;
-    const real B2_half = (w1 * sqrt_det_h(m, p_mH0) * beta1(m, p_mH0) * BB(i1 - 1, i2, 4) +
-                          w2 * sqrt_det_h(m, p_pH0) * beta1(m, p_pH0) * BB(i1, i2, 4)) / ww;
-    w1 = sqrt_det_h_tilde(m, p_mHpH), w2 = sqrt_det_h_tilde(m, p_pHpH);
-    ww = (real)2 * sqrt_det_h_tilde(m, p_0pH);
-    const real B3_half = (w1 * sqrt_det_h(m, p_mHpH) * beta1(m, p_mHpH) * BB(i1 - 1, i2, 5) +
-                          w2 * sqrt_det_h(m, p_pHpH) * beta1(m, p_pHpH) * BB(i1, i2, 5)) / ww;
-    w1 = sqrt_det_h_tilde(m, p_00), w2 = sqrt_det_h_tilde(m, p_10);
-    ww = (real)2 * sqrt_det_h_tilde(m, p_pH0);
-    const real D3_half = (w1 * h_13(m, p_00) * DD(i1, i2, 2) + w2 * h_13(m, p_10) * DD(i1 + 1, i2, 2)) / ww;
-    const real D1_cov = h_11(m, p_pH0) * DD(i1, i2, 0) + D3_half;
-    const real D2_cov = h_22(m, p_0pH) * DD(i1, i2, 1);
-    const real D3_cov = h_33(m, p_00) * DD(i1, i2, 2) + D1_half;
+  int             i2 = 0;
+  QRow<real>      r0, rH;
+  row_spans<30>(R, [&](int j) {
+    i2 = j;
+    r0 = qrow(m, (real)(i2 - f.ng)), rH = qrow(m, (real)(i2 - f.ng) + H);
+  }, [&](int i1, int lane) {
+    const bool       in  = i1 <= R.i1;  // the cells of R and one on either side
+    const real       i1_ = (real)(i1 - f.ng);
+    const QCol<real> c0 = qcol(m, i1_), cH = qcol(m, i1_ + H);
+    const QPt<real>  p_00 = qpt(m, c0, r0), p_pH0 = qpt(m, cH, r0);
+    const QPt<real>  p_0pH = qpt(m, c0, rH), p_pHpH = qpt(m, cH, rH);
+    auto             ld = [&](const FieldView<real>& F, int c) { return in ? F.p[F.idx(i1, i2, 0, c)] : (real)0; };
+    const real D1 = ld(Df, 0), D3 = ld(Df, 2);
+    const real w_pH0 = sqrt_det_h_tilde(m, p_pH0), w_pHpH = sqrt_det_h_tilde(m, p_pHpH);
+    const real w_00 = sqrt_det_h_tilde(m, p_00), w_0pH = sqrt_det_h_tilde(m, p_0pH);
+    const real d1 = w_pH0 * h_13(m, p_pH0) * D1;
+    const real b2 = w_pH0 * sqrt_det_h(m, p_pH0) * beta1(m, p_pH0) * ld(Bf, 4);
+    const real b3 = w_pHpH * sqrt_det_h(m, p_pHpH) * beta1(m, p_pHpH) * ld(Bf, 5);
+    const real d3 = w_00 * h_13(m, p_00) * D3;
+    const real d1m = __shfl_up_sync(0xffffffffu, d1, 1), b2m = __shfl_up_sync(0xffffffffu, b2, 1);
+    const real b3m = __shfl_up_sync(0xffffffffu, b3, 1), d3p = __shfl_down_sync(0xffffffffu, d3, 1);
+    if (lane == 0 || lane == 31 || i1 >= R.i1) return;
+    const real D1_half = (d1m + d1) / ((real)2 * w_00);
+    const real B2_half = (b2m + b2) / ((real)2 * w_00);
+    const real B3_half = (b3m + b3) / ((real)2 * w_0pH);
+    const real D3_half = (d3 + d3p) / ((real)2 * w_pH0);
+    const real D1_cov = h_11(m, p_pH0) * D1 + D3_half;
+    const real D2_cov = h_22(m, p_0pH) * Df.p[Df.idx(i1, i2, 0, 1)];
+    const real D3_cov = h_33(m, p_00) * D3 + D1_half;
     Ef.p[Ef.idx(i1, i2, 0, 0)] = alpha(m, p_pH0) * D1_cov;
     Ef.p[Ef.idx(i1, i2, 0, 1)] = alpha(m, p_0pH) * D2_cov - B3_half;
     Ef.p[Ef.idx(i1, i2, 0, 2)] = alpha(m, p_00) * D3_cov + B2_half;
-#undef DD
-#undef BB
-  }
+  });
 }
 
-// ComputeAuxH_kernel (aux_fields_gr.hpp:131-193)
+// ComputeAuxH_kernel (aux_fields_gr.hpp:131-193), as k_gr_aux_e (24 and 15 us)
 template <typename real>
-__global__ void k_gr_aux_h(GRFld<real> f, Range2 R, FieldView<real> Df, FieldView<real> Bf,
-                           FieldView<real> Hf) {
+__global__ void __launch_bounds__(128) k_gr_aux_h(GRFld<real> f, Range2 R, FieldView<real> Df,
+                                                  FieldView<real> Bf, FieldView<real> Hf) {
   const QKS<real> m = f.m.template as<real>();
   const real      H = 0.5;
-  GR_CELL_LOOP(R)
-    const real i1_ = (real)(i1 - f.ng), i2_ = (real)(i2 - f.ng);
-#define DD(a, b, c) Df.p[Df.idx(a, b, 0, c)]
-#define BB(a, b, c) Bf.p[Bf.idx(a, b, 0, c)]
-    const QPt<real> p_0pH = qpt(m, i1_, i2_ + H), p_pH0 = qpt(m, i1_ + H, i2_);
-    const QPt<real> p_pHpH = qpt(m, i1_ + H, i2_ + H), p_1pH = qpt(m, i1_ + (real)1, i2_ + H);
-    const QPt<real> p_00 = qpt(m, i1_, i2_), p_10 = qpt(m, i1_ + (real)1, i2_);
-    const QPt<real> p_mHpH = qpt(m, i1_ - H, i2_ + H);
-    real w1 = sqrt_det_h_tilde(m, p_0pH), w2 = sqrt_det_h_tilde(m, p_1pH);
-    real ww = (real)2 * sqrt_det_h_tilde(m, p_pHpH);
-    const real B1_half = (w1 * h_13(m, p_0pH) * BB(i1, i2, 3) + w2 * h_13(m, p_1pH) * BB(i1 + 1, i2, 3)) / ww;
-    const real D2_half = (w1 * sqrt_det_h(m, p_0pH) * beta1(m, p_0pH) * DD(i1, i2, 1) +
-                          w2 * sqrt_det_h(m, p_1pH) * beta1(m, p_1pH) * DD(i1 + 1, i2, 1)) / ww;
-    w1 = sqrt_det_h_tilde(m, p_00), w2 = sqrt_det_h_tilde(m, p_10);
-    ww = (real)2 * sqrt_det_h_tilde(m, p_pH0);
-    const real D3_half = (w1 * sqrt_det_h(m, p_00) * beta1(m, p_00) * DD(i1, i2, 2) +
-                          w2 * sqrt_det_h(m, p_10) * beta1(m, p_10) * DD(i1 + 1, i2, 2)) / ww;
-    w1 = sqrt_det_h_tilde(m, p_mHpH), w2 = sqrt_det_h_tilde(m, p_pHpH);
-    ww = (real)2 * sqrt_det_h_tilde(m, p_0pH);
-    const real B3_half = (w1 * h_13(m, p_mHpH) * BB(i1 - 1, i2, 5) + w2 * h_13(m, p_pHpH) * BB(i1, i2, 5)) / ww;
-    const real B1_cov = h_11(m, p_0pH) * BB(i1, i2, 3) + B3_half;
-    const real B2_cov = h_22(m, p_pH0) * BB(i1, i2, 4);
-    const real B3_cov = h_33(m, p_pHpH) * BB(i1, i2, 5) + B1_half;
+  int             i2 = 0;
+  QRow<real>      r0, rH;
+  row_spans<30>(R, [&](int j) {
+    i2 = j;
+    r0 = qrow(m, (real)(i2 - f.ng)), rH = qrow(m, (real)(i2 - f.ng) + H);
+  }, [&](int i1, int lane) {
+    const bool       in  = i1 <= R.i1;
+    const real       i1_ = (real)(i1 - f.ng);
+    const QCol<real> c0 = qcol(m, i1_), cH = qcol(m, i1_ + H);
+    const QPt<real>  p_00 = qpt(m, c0, r0), p_pH0 = qpt(m, cH, r0);
+    const QPt<real>  p_0pH = qpt(m, c0, rH), p_pHpH = qpt(m, cH, rH);
+    auto             ld = [&](const FieldView<real>& F, int c) { return in ? F.p[F.idx(i1, i2, 0, c)] : (real)0; };
+    const real B1 = ld(Bf, 3), B3 = ld(Bf, 5);
+    const real w_pH0 = sqrt_det_h_tilde(m, p_pH0), w_pHpH = sqrt_det_h_tilde(m, p_pHpH);
+    const real w_00 = sqrt_det_h_tilde(m, p_00), w_0pH = sqrt_det_h_tilde(m, p_0pH);
+    const real b1 = w_0pH * h_13(m, p_0pH) * B1;
+    const real d2 = w_0pH * sqrt_det_h(m, p_0pH) * beta1(m, p_0pH) * ld(Df, 1);
+    const real d3 = w_00 * sqrt_det_h(m, p_00) * beta1(m, p_00) * ld(Df, 2);
+    const real b3 = w_pHpH * h_13(m, p_pHpH) * B3;
+    const real b1p = __shfl_down_sync(0xffffffffu, b1, 1), d2p = __shfl_down_sync(0xffffffffu, d2, 1);
+    const real d3p = __shfl_down_sync(0xffffffffu, d3, 1), b3m = __shfl_up_sync(0xffffffffu, b3, 1);
+    if (lane == 0 || lane == 31 || i1 >= R.i1) return;
+    const real B1_half = (b1 + b1p) / ((real)2 * w_pHpH);
+    const real D2_half = (d2 + d2p) / ((real)2 * w_pHpH);
+    const real D3_half = (d3 + d3p) / ((real)2 * w_pH0);
+    const real B3_half = (b3m + b3) / ((real)2 * w_0pH);
+    const real B1_cov = h_11(m, p_0pH) * B1 + B3_half;
+    const real B2_cov = h_22(m, p_pH0) * Bf.p[Bf.idx(i1, i2, 0, 4)];
+    const real B3_cov = h_33(m, p_pHpH) * B3 + B1_half;
     Hf.p[Hf.idx(i1, i2, 0, 3)] = alpha(m, p_0pH) * B1_cov;
     Hf.p[Hf.idx(i1, i2, 0, 4)] = alpha(m, p_pH0) * B2_cov + D3_half;
     Hf.p[Hf.idx(i1, i2, 0, 5)] = alpha(m, p_pHpH) * B3_cov - D2_half;
-#undef DD
-#undef BB
-  }
+  });
 }
 
 // TimeAverageDB / TimeAverageJ (aux_fields_gr.hpp:222-280)
@@ -723,12 +778,14 @@ __global__ void k_gr_horizon(GRFld<real> f, FieldView<real> F, int set_e, int se
   const int i2 = f.ng + blockIdx.x * blockDim.x + threadIdx.x;
   if (i2 >= f.n2 + f.ng + 1) return;
   const int i1min = f.ng, src = i1min + 1 + nfilter;
+  // the source cell lies past the cells written, or is one of them
+  real v[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) v[c] = (c < 3 ? set_e : set_b) ? F.p[F.idx(src, i2, 0, c)] : (real)0;
   for (int i = 0; i <= 2 + nfilter; ++i) {
-    const int dst = i1min - f.ng + i;
-    if (set_e)
-      for (int c = 0; c < 3; ++c) F.p[F.idx(dst, i2, 0, c)] = F.p[F.idx(src, i2, 0, c)];
-    if (set_b)
-      for (int c = 3; c < 6; ++c) F.p[F.idx(dst, i2, 0, c)] = F.p[F.idx(src, i2, 0, c)];
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+      if (c < 3 ? set_e : set_b) F.p[F.idx(i, i2, 0, c)] = v[c];
   }
 }
 
@@ -873,6 +930,13 @@ pic::GRFld<real> fld_of(const pic_ctx* c, const pic_gr_metric* g) {
   f.axis_min = g->axis_min;
   f.axis_max = g->axis_max;
   return f;
+}
+
+// blocks of 128 threads for row_spans<W> over R
+unsigned row_blocks(const pic::Range2& R, int W) {
+  const int64_t spans  = (R.i1 - R.i0 + W - 1) / W;
+  const int64_t groups = (spans + pic::kRowChunks - 1) / pic::kRowChunks;
+  return (unsigned)std::max<int64_t>((groups * (R.j1 - R.j0) + 3) / 4, 1);
 }
 
 unsigned blocks_for(int64_t n) {
@@ -1163,12 +1227,12 @@ int pic_gr_faraday(pic_ctx* c, const pic_gr_metric* g, const void* Bin, void* Bo
   if (!Bin || !Bout || !E) return PIC_ERR_ARG;
   cudaStream_t      s = strm(stream);
   const pic::Range2 R = active(c);
-  const unsigned    b = blocks_for((int64_t)c->grid.n[0] * c->grid.n[1]);
+  const unsigned    b = row_blocks(R, 32);
   GR_FLD_DISPATCH(
-    PIC_KL(pic::k_gr_faraday<float><<<b, 256, 0, s>>>(fld_of<float>(c, g), R, em_view<float>(c, Bin),
+    PIC_KL(pic::k_gr_faraday<float><<<b, 128, 0, s>>>(fld_of<float>(c, g), R, em_view<float>(c, Bin),
                                                       em_view<float>(c, Bout), em_view<float>(c, E),
                                                       (float)coeff)),
-    PIC_KL(pic::k_gr_faraday<double><<<b, 256, 0, s>>>(fld_of<double>(c, g), R, em_view<double>(c, Bin),
+    PIC_KL(pic::k_gr_faraday<double><<<b, 128, 0, s>>>(fld_of<double>(c, g), R, em_view<double>(c, Bin),
                                                        em_view<double>(c, Bout), em_view<double>(c, E),
                                                        coeff)))
 }
@@ -1182,18 +1246,18 @@ int pic_gr_ampere(pic_ctx* c, const pic_gr_metric* g, const void* Din, void* Dou
   const int    ng = c->grid.ng;
   // ampere range: i2 in [i2min, i2max + 1) (fieldsolvers.h:180-182)
   const pic::Range2 R{ ng, c->grid.n[0] + ng, ng, c->grid.n[1] + ng + 1 };
-  const unsigned    b  = blocks_for((int64_t)c->grid.n[0] * (c->grid.n[1] + 1));
+  const unsigned    b  = row_blocks(R, 32);
   const unsigned    ba = (unsigned)((c->grid.n[0] + 255) / 256);
   const bool        alias = Din == Dout;
   if (is_f64(c)) {
     const auto f = fld_of<double>(c, g);
-    PIC_KL(pic::k_gr_ampere<double><<<b, 256, 0, s>>>(f, R, em_view<double>(c, Din), em_view<double>(c, Dout),
+    PIC_KL(pic::k_gr_ampere<double><<<b, 128, 0, s>>>(f, R, em_view<double>(c, Din), em_view<double>(c, Dout),
                                                       em_view<double>(c, H), coeff));
     PIC_KL(pic::k_gr_ampere_axis<double><<<ba, 256, 0, s>>>(f, em_view<double>(c, Din),
                                                             em_view<double>(c, Dout), alias));
   } else {
     const auto f = fld_of<float>(c, g);
-    PIC_KL(pic::k_gr_ampere<float><<<b, 256, 0, s>>>(f, R, em_view<float>(c, Din), em_view<float>(c, Dout),
+    PIC_KL(pic::k_gr_ampere<float><<<b, 128, 0, s>>>(f, R, em_view<float>(c, Din), em_view<float>(c, Dout),
                                                      em_view<float>(c, H), (float)coeff));
     PIC_KL(pic::k_gr_ampere_axis<float><<<ba, 256, 0, s>>>(f, em_view<float>(c, Din),
                                                            em_view<float>(c, Dout), alias));
@@ -1209,11 +1273,11 @@ int pic_gr_currents_ampere(pic_ctx* c, const pic_gr_metric* g, void* D, const vo
   cudaStream_t      s  = strm(stream);
   const int         ng = c->grid.ng;
   const pic::Range2 R{ ng, c->grid.n[0] + ng, ng, c->grid.n[1] + ng + 1 };
-  const unsigned    b = blocks_for((int64_t)c->grid.n[0] * (c->grid.n[1] + 1));
+  const unsigned    b = row_blocks(R, 32);
   GR_FLD_DISPATCH(
-    PIC_KL(pic::k_gr_currents_ampere<float><<<b, 256, 0, s>>>(fld_of<float>(c, g), R, em_view<float>(c, D),
+    PIC_KL(pic::k_gr_currents_ampere<float><<<b, 128, 0, s>>>(fld_of<float>(c, g), R, em_view<float>(c, D),
                                                               cur_view<float>(c, J), (float)coeff)),
-    PIC_KL(pic::k_gr_currents_ampere<double><<<b, 256, 0, s>>>(fld_of<double>(c, g), R, em_view<double>(c, D),
+    PIC_KL(pic::k_gr_currents_ampere<double><<<b, 128, 0, s>>>(fld_of<double>(c, g), R, em_view<double>(c, D),
                                                                cur_view<double>(c, J), coeff)))
 }
 
@@ -1226,15 +1290,15 @@ int pic_gr_aux(pic_ctx* c, const pic_gr_metric* g, int32_t which, const void* D,
   const int    ng = c->grid.ng;
   // range_with_axis_BCs (fieldsolvers.h:58-81)
   const pic::Range2 R{ ng - 1, c->grid.n[0] + ng, ng, c->grid.n[1] + ng + (g->axis_max ? 1 : 0) };
-  const unsigned    b = blocks_for((int64_t)(c->grid.n[0] + 1) * (c->grid.n[1] + 1));
+  const unsigned    b = row_blocks(R, 30);
   if (is_f64(c)) {
     const auto f = fld_of<double>(c, g);
-    if (which == 0) PIC_KL(pic::k_gr_aux_e<double><<<b, 256, 0, s>>>(f, R, em_view<double>(c, D), em_view<double>(c, B), em_view<double>(c, out)));
-    else            PIC_KL(pic::k_gr_aux_h<double><<<b, 256, 0, s>>>(f, R, em_view<double>(c, D), em_view<double>(c, B), em_view<double>(c, out)));
+    if (which == 0) PIC_KL(pic::k_gr_aux_e<double><<<b, 128, 0, s>>>(f, R, em_view<double>(c, D), em_view<double>(c, B), em_view<double>(c, out)));
+    else            PIC_KL(pic::k_gr_aux_h<double><<<b, 128, 0, s>>>(f, R, em_view<double>(c, D), em_view<double>(c, B), em_view<double>(c, out)));
   } else {
     const auto f = fld_of<float>(c, g);
-    if (which == 0) PIC_KL(pic::k_gr_aux_e<float><<<b, 256, 0, s>>>(f, R, em_view<float>(c, D), em_view<float>(c, B), em_view<float>(c, out)));
-    else            PIC_KL(pic::k_gr_aux_h<float><<<b, 256, 0, s>>>(f, R, em_view<float>(c, D), em_view<float>(c, B), em_view<float>(c, out)));
+    if (which == 0) PIC_KL(pic::k_gr_aux_e<float><<<b, 128, 0, s>>>(f, R, em_view<float>(c, D), em_view<float>(c, B), em_view<float>(c, out)));
+    else            PIC_KL(pic::k_gr_aux_h<float><<<b, 128, 0, s>>>(f, R, em_view<float>(c, D), em_view<float>(c, B), em_view<float>(c, out)));
   }
   return cuda_status(cudaGetLastError());
 }

@@ -73,16 +73,37 @@ struct QPt {
   M chi, ex, r, eta, th, s, c, dtde, Sg, Dl, A, z;
 };
 
+// the quantities of an x1 and of an x2 alone
 template <typename M>
-__device__ __forceinline__ QPt<M> qpt(const QKS<M>& m, M x1, M x2) {
+struct QCol {
+  M chi, ex, r;
+};
+template <typename M>
+struct QRow {
+  M eta, th, s, c, dtde;
+};
+template <typename M>
+__device__ __forceinline__ QCol<M> qcol(const QKS<M>& m, M x1) {
+  QCol<M> q;
+  q.chi = x1 * m.dchi + m.chi_min;
+  q.ex  = mexp(q.chi);
+  q.r   = m.r0 + q.ex;
+  return q;
+}
+template <typename M>
+__device__ __forceinline__ QRow<M> qrow(const QKS<M>& m, M x2) {
+  QRow<M> q;
+  q.eta = x2 * m.deta + m.eta_min;
+  q.th  = m.eta2theta(q.eta);
+  msincos(q.th, &q.s, &q.c);
+  q.dtde = m.dtheta_deta(q.eta);
+  return q;
+}
+template <typename M>
+__device__ __forceinline__ QPt<M> qpt(const QKS<M>& m, const QCol<M>& u, const QRow<M>& v) {
   QPt<M> p;
-  p.chi  = x1 * m.dchi + m.chi_min;
-  p.ex   = mexp(p.chi);
-  p.r    = m.r0 + p.ex;
-  p.eta  = x2 * m.deta + m.eta_min;
-  p.th   = m.eta2theta(p.eta);
-  msincos(p.th, &p.s, &p.c);
-  p.dtde = m.dtheta_deta(p.eta);
+  p.chi = u.chi, p.ex = u.ex, p.r = u.r;
+  p.eta = v.eta, p.th = v.th, p.s = v.s, p.c = v.c, p.dtde = v.dtde;
   const M a2 = m.a * m.a;
   p.Sg = p.r * p.r + a2 * (p.c * p.c);
   p.Dl = p.r * p.r - (M)2 * p.r + a2;
@@ -90,6 +111,10 @@ __device__ __forceinline__ QPt<M> qpt(const QKS<M>& m, M x1, M x2) {
   p.A  = rr * rr - a2 * p.Dl * (p.s * p.s);
   p.z  = (M)2 * p.r / p.Sg;
   return p;
+}
+template <typename M>
+__device__ __forceinline__ QPt<M> qpt(const QKS<M>& m, M x1, M x2) {
+  return qpt(m, qcol(m, x1), qrow(m, x2));
 }
 
 // h_ij (qkerr_schild.h:145-188), h^ij (194-233)

@@ -1,10 +1,10 @@
 """The FP64 island's push (its own formulas on the device) and the early end of
 the geodesic passes, against the oracle's double-precision push of the same
-FP32 particles."""
+FP32 particles; the GR field kernels at the remainders of their rows."""
 import pytest
 import torch
 
-from tests.test_gpu_gr import _particles, _rand_fields, _setup, _X
+from tests.test_gpu_gr import TOL, _particles, _rand_fields, _setup, _X
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +34,33 @@ def test_island_push(order, h, pusher, dt, niter):
         a, b = sp.u[c].double()[ok], spg.u[c].cpu().double()[ok]
         assert bool(torch.isfinite(a).all())
         assert float((a - b).abs().max()) <= 2.0 ** -22 * float(a.abs().max())
+
+
+@pytest.mark.parametrize("real", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n", [(4, 8), (29, 9), (30, 16), (31, 12), (61, 10), (128, 24)])
+def test_field_rows(n, real):
+    """The field kernels' rows of 30 and 32 cells, one and several per warp, at
+    their remainders, against the oracle."""
+    from entity_gb300.inputs import empty_field
+    g, spec, ctx, o = _setup(real, order=2, n=n)
+    em, J = _rand_fields(g, 3), _rand_fields(g, 4)[:3].clone()
+    emg, Jg = em.cuda(), J.cuda()
+
+    def same(a, b, what):  # the bound of the field kernels' parity (test_gpu_gr)
+        torch.cuda.synchronize()
+        assert float((a - b.cpu()).abs().max()) <= 10 * TOL[real] * float(a.abs().max()), what
+
+    for which, ref in enumerate((o.gr_aux_e, o.gr_aux_h)):
+        a, b = empty_field(g, 6), empty_field(g, 6, "cuda")
+        ref(em, em, a)
+        ctx.gr_aux(which, emg, emg, b)
+        same(a, b, which)
+    for name in ("gr_faraday", "gr_ampere"):
+        a, b = em.clone(), emg.clone()
+        getattr(o, name)(em, a, em, 0.01)
+        getattr(ctx, name)(emg, b, emg, 0.01)
+        same(a, b, name)
+    a, b = em.clone(), emg.clone()
+    o.gr_currents_ampere(a, J, 0.01)
+    ctx.gr_currents_ampere(b, Jg, 0.01)
+    same(a, b, "currents")
