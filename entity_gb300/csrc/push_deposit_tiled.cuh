@@ -445,10 +445,18 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
   const JWinFixed<G, FA>   add_fixed{ Jw, jb };
   const JWinReal<G, real> add_real{ Jr, jb };
 
-  // 2. particles of the tile, species by species; with records in chunks,
-  //    each pushed by the whole CTA and then deposited
+  // 2. particles of the tile (this CTA's part of them), species by species;
+  //    with records in chunks, each pushed by the whole CTA and then deposited
+  auto part = [&](int k, unsigned y) -> int64_t {
+    const int32_t* ts = a.s[k].tile_start + t;
+    if (gridDim.y == 1) return ts[y - blockIdx.y];
+    // whole groups of 128 particles, the largest lane-strided group
+    const unsigned n   = (unsigned)(ts[1] - ts[0]);
+    const unsigned len = ((n + gridDim.y - 1) / gridDim.y + 127u) & ~127u;
+    return ts[0] + (int64_t)min((uint64_t)n, (uint64_t)len * y);
+  };
   int     s  = 0;
-  int64_t p0 = a.s[0].tile_start[t];  // first particle of the CTA's next group
+  int64_t p0 = part(0, blockIdx.y);  // first particle of the CTA's next group
   for (;;) {
     int pend = 0;  // particles since the last deposit, rounded up to groups
     while (s < a.nsp) {
@@ -459,7 +467,7 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
       int32_t*       ipa[3] = { S.sp.i1p, S.sp.i2p, S.sp.i3p };
       float*         da[3]  = { S.sp.dx1, S.sp.dx2, S.sp.dx3 };
       float*         dpa[3] = { S.sp.dx1p, S.sp.dx2p, S.sp.dx3p };
-      const int64_t  hi = S.tile_start[t + 1];
+      const int64_t  hi = part(s, blockIdx.y + 1);
       for (; p0 < hi && (!REC || pend + NT <= G::CHUNK); p0 += NT, pend += NT) {
         const int64_t p = p0 + local;
         if (p >= hi) continue;
@@ -608,7 +616,7 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
         }
       }
       if (p0 < hi) break;  // the chunk is full
-      if (++s < a.nsp) p0 = a.s[s].tile_start[t];
+      if (++s < a.nsp) p0 = part(s, blockIdx.y);
     }
     __syncthreads();
     if constexpr (REC) {
