@@ -2,7 +2,8 @@
 // Ampere Yee updates, the J -> E coupling, the periodic current fold, the
 // digital current filter and ghost exchange, and the FP64 energy reduction.
 //
-// Every kernel maps one thread to one active cell (i1 fastest) and, where the
+// The update kernels map one thread to one active cell (i1 fastest; the fold and
+// the ghost fill visit the cells near periodic edges only) and, where the
 // reference follows the update with a periodic CommunicateFields, writes the
 // cell's new value straight into its ghost images as well, which removes the
 // reference's separate halo pass (src/framework/domain/comm_nompi.hpp:44-63).
