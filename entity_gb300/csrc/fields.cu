@@ -4,7 +4,7 @@
 //
 // The update kernels map one thread to one active cell (i1 fastest; the fold and
 // the ghost fill visit the cells near periodic edges only) and, where the
-// reference follows the update with a periodic CommunicateFields, writes the
+// reference follows the update with a periodic CommunicateFields, write the
 // cell's new value straight into its ghost images as well, which removes the
 // reference's separate halo pass (src/framework/domain/comm_nompi.hpp:44-63).
 #include <algorithm>

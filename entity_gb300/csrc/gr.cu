@@ -449,6 +449,13 @@ struct GRFld {
   int             ng, n1, n2, axis_min, axis_max;
 };
 
+// one or two fields of a boundary launch, by blockIdx.y (a step's boundaries act
+// on em and em0 alike: 24 launches of 3 us in a Wald step of 604 us, 12 in 538)
+template <typename real>
+struct Pair {
+  FieldView<real> f[2];
+};
+
 // Faraday_kernel (faraday_gr.hpp:62-90): Bout = Bin + coeff curl E. Bound by
 // the metric's divisions and roots, like the four kernels below; 1024 x 512
 // cells: 12.7 us with every cell's own sines and cosines, 11.5 us.
@@ -737,7 +744,8 @@ __global__ void k_gr_filter(GRFld<real> f, Range2 R, FieldView<real> A, FieldVie
 
 // AxisBoundaries_kernel (fields_bcs.hpp:825-868), per i1 over all cells
 template <typename real>
-__global__ void k_gr_axis(GRFld<real> f, FieldView<real> F, int set_e, int set_b) {
+__global__ void k_gr_axis(GRFld<real> f, const __grid_constant__ Pair<real> P, int set_e, int set_b) {
+  const FieldView<real>& F = P.f[blockIdx.y];
   const int i1 = blockIdx.x * blockDim.x + threadIdx.x;
   if (i1 >= f.n1 + 2 * f.ng) return;
 #define FF(j, c) F.p[F.idx(i1, j, 0, c)]
@@ -774,7 +782,8 @@ __global__ void k_gr_axis(GRFld<real> f, FieldView<real> F, int set_e, int set_b
 
 // HorizonBoundaries_kernel (fields_bcs.hpp:1188-1240), per i2
 template <typename real>
-__global__ void k_gr_horizon(GRFld<real> f, FieldView<real> F, int set_e, int set_b, int nfilter) {
+__global__ void k_gr_horizon(GRFld<real> f, const __grid_constant__ Pair<real> P, int set_e, int set_b, int nfilter) {
+  const FieldView<real>& F = P.f[blockIdx.y];
   const int i2 = f.ng + blockIdx.x * blockDim.x + threadIdx.x;
   if (i2 >= f.n2 + f.ng + 1) return;
   const int i1min = f.ng, src = i1min + 1 + nfilter;
@@ -796,8 +805,9 @@ __global__ void k_gr_horizon(GRFld<real> f, FieldView<real> F, int set_e, int se
 // radius (i + 1/2 for D^r, B^theta, B^phi; i for D^theta, D^phi, B^r). On
 // the axis rows D^phi only decays (its target term is skipped there).
 template <typename real>
-__global__ void k_gr_match(GRFld<real> f, Range2 R, FieldView<real> F, FieldView<real> T,
-                           real r_edge, real ds, int set_e, int set_b) {
+__global__ void k_gr_match(GRFld<real> f, Range2 R, const __grid_constant__ Pair<real> P,
+                           FieldView<real> T, real r_edge, real ds, int set_e, int set_b) {
+  const FieldView<real>& F = P.f[blockIdx.y];
   const QKS<real> m = f.m.template as<real>();
   const real      H = 0.5, ONE = 1, FOUR = 4;
   const int       N2 = f.n2 + 2 * f.ng;
@@ -1156,7 +1166,77 @@ pic::Range2 match_range(const pic_ctx* c, const pic_gr_metric* g, double ds) {
   return pic::Range2{ i0, std::max(i0, i1), 0, c->grid.n[1] + 2 * ng };
 }
 
+template <typename real>
+pic::Pair<real> pair_of(const pic_ctx* c, void* const* f, int n) {
+  return { { em_view<real>(c, f[0]), em_view<real>(c, f[n - 1]) } };
+}
+
+// pic_gr_field_bcs on n (1 or 2) fields
+int gr_field_bcs(pic_ctx* c, const pic_gr_metric* g, void* const* fld, int n, int32_t set_e,
+                 int32_t set_b, int32_t nfilter, void* stream) {
+  int st = gr_check(c, g);
+  if (st != PIC_OK) return st;
+  if (!fld[0] || !fld[n - 1] || nfilter < 0) return PIC_ERR_ARG;
+  cudaStream_t s = strm(stream);
+  const dim3   b1((unsigned)((c->grid.n[0] + 2 * c->grid.ng + 255) / 256), (unsigned)n);
+  const dim3   b2((unsigned)((c->grid.n[1] + 1 + 255) / 256), (unsigned)n);
+  if (is_f64(c)) {
+    const auto f = fld_of<double>(c, g);
+    const auto P = pair_of<double>(c, fld, n);
+    if (g->horizon) PIC_KL(pic::k_gr_horizon<double><<<b2, 256, 0, s>>>(f, P, set_e, set_b, nfilter));
+    if (g->axis_min || g->axis_max) PIC_KL(pic::k_gr_axis<double><<<b1, 256, 0, s>>>(f, P, set_e, set_b));
+  } else {
+    const auto f = fld_of<float>(c, g);
+    const auto P = pair_of<float>(c, fld, n);
+    if (g->horizon) PIC_KL(pic::k_gr_horizon<float><<<b2, 256, 0, s>>>(f, P, set_e, set_b, nfilter));
+    if (g->axis_min || g->axis_max) PIC_KL(pic::k_gr_axis<float><<<b1, 256, 0, s>>>(f, P, set_e, set_b));
+  }
+  return cuda_status(cudaGetLastError());
+}
+
+// pic_gr_match_fields on n (1 or 2) fields
+int gr_match_fields(pic_ctx* c, const pic_gr_metric* g, void* const* fld, int n, const void* target,
+                    double ds, int32_t set_e, int32_t set_b, void* stream) {
+  int st = gr_check(c, g);
+  if (st != PIC_OK) return st;
+  if (!fld[0] || !fld[n - 1] || !target || !(ds > 0.0)) return PIC_ERR_ARG;
+  cudaStream_t s = strm(stream);
+  if (is_f64(c)) {
+    const auto R = match_range<double>(c, g, ds);
+    if (R.count() == 0) return PIC_OK;
+    PIC_KL(pic::k_gr_match<double><<<dim3(blocks_for(R.count()), (unsigned)n), 256, 0, s>>>(
+      fld_of<double>(c, g), R, pair_of<double>(c, fld, n), em_view<double>(c, target),
+      (double)g->x1max, ds, set_e, set_b));
+  } else {
+    const auto R = match_range<float>(c, g, ds);
+    if (R.count() == 0) return PIC_OK;
+    PIC_KL(pic::k_gr_match<float><<<dim3(blocks_for(R.count()), (unsigned)n), 256, 0, s>>>(
+      fld_of<float>(c, g), R, pair_of<float>(c, fld, n), em_view<float>(c, target),
+      (float)g->x1max, (float)ds, set_e, set_b));
+  }
+  return cuda_status(cudaGetLastError());
+}
+
 }  // namespace
+
+namespace pic_internal {
+int gr_boundaries(pic_ctx* c, const pic_gr_metric* g, void* const* fld, const void* target,
+                  double ds, int32_t set_e, int32_t set_b, int32_t nfilter, void* stream) {
+  // two views of one array would be written by two blocks at once
+  if (fld[0] == fld[1]) {
+    for (int k = 0; k < 2; ++k) {
+      int st = gr_field_bcs(c, g, fld + k, 1, set_e, set_b, nfilter, stream);
+      if (st == PIC_OK && ds > 0.0)
+        st = gr_match_fields(c, g, fld + k, 1, target, ds, set_e, set_b, stream);
+      if (st != PIC_OK) return st;
+    }
+    return PIC_OK;
+  }
+  const int st = gr_field_bcs(c, g, fld, 2, set_e, set_b, nfilter, stream);
+  if (st != PIC_OK || !(ds > 0.0)) return st;
+  return gr_match_fields(c, g, fld, 2, target, ds, set_e, set_b, stream);
+}
+}  // namespace pic_internal
 
 extern "C" {
 
@@ -1357,44 +1437,14 @@ int pic_gr_filter_currents(pic_ctx* c, const pic_gr_metric* g, void* J, void* bu
 // horizon's copies in the corner cells
 int pic_gr_field_bcs(pic_ctx* c, const pic_gr_metric* g, void* fld, int32_t set_e, int32_t set_b,
                      int32_t nfilter, void* stream) {
-  int st = gr_check(c, g);
-  if (st != PIC_OK) return st;
-  if (!fld || nfilter < 0) return PIC_ERR_ARG;
-  cudaStream_t   s  = strm(stream);
-  const unsigned b1 = (unsigned)((c->grid.n[0] + 2 * c->grid.ng + 255) / 256);
-  const unsigned b2 = (unsigned)((c->grid.n[1] + 1 + 255) / 256);
-  if (is_f64(c)) {
-    const auto f = fld_of<double>(c, g);
-    if (g->horizon) PIC_KL(pic::k_gr_horizon<double><<<b2, 256, 0, s>>>(f, em_view<double>(c, fld), set_e, set_b, nfilter));
-    if (g->axis_min || g->axis_max) PIC_KL(pic::k_gr_axis<double><<<b1, 256, 0, s>>>(f, em_view<double>(c, fld), set_e, set_b));
-  } else {
-    const auto f = fld_of<float>(c, g);
-    if (g->horizon) PIC_KL(pic::k_gr_horizon<float><<<b2, 256, 0, s>>>(f, em_view<float>(c, fld), set_e, set_b, nfilter));
-    if (g->axis_min || g->axis_max) PIC_KL(pic::k_gr_axis<float><<<b1, 256, 0, s>>>(f, em_view<float>(c, fld), set_e, set_b));
-  }
-  return cuda_status(cudaGetLastError());
+  void* f[1] = { fld };
+  return gr_field_bcs(c, g, f, 1, set_e, set_b, nfilter, stream);
 }
 
 int pic_gr_match_fields(pic_ctx* c, const pic_gr_metric* g, void* fld, const void* target,
                         double ds, int32_t set_e, int32_t set_b, void* stream) {
-  int st = gr_check(c, g);
-  if (st != PIC_OK) return st;
-  if (!fld || !target || !(ds > 0.0)) return PIC_ERR_ARG;
-  cudaStream_t s = strm(stream);
-  if (is_f64(c)) {
-    const auto R = match_range<double>(c, g, ds);
-    if (R.count() == 0) return PIC_OK;
-    PIC_KL(pic::k_gr_match<double><<<blocks_for(R.count()), 256, 0, s>>>(
-      fld_of<double>(c, g), R, em_view<double>(c, fld), em_view<double>(c, target),
-      (double)g->x1max, ds, set_e, set_b));
-  } else {
-    const auto R = match_range<float>(c, g, ds);
-    if (R.count() == 0) return PIC_OK;
-    PIC_KL(pic::k_gr_match<float><<<blocks_for(R.count()), 256, 0, s>>>(
-      fld_of<float>(c, g), R, em_view<float>(c, fld), em_view<float>(c, target),
-      (float)g->x1max, (float)ds, set_e, set_b));
-  }
-  return cuda_status(cudaGetLastError());
+  void* f[1] = { fld };
+  return gr_match_fields(c, g, f, 1, target, ds, set_e, set_b, stream);
 }
 
 int pic_gr_absorb_currents(pic_ctx* c, const pic_gr_metric* g, void* J, double ds, void* stream) {

@@ -11,6 +11,12 @@
 #include "../../include/entity_pic.h"
 #include "srpic_engine.hpp"
 
+namespace pic_internal {
+// pic_gr_field_bcs, and pic_gr_match_fields for ds > 0, on fld[0] and fld[1] (csrc/gr.cu)
+int gr_boundaries(pic_ctx* c, const pic_gr_metric* g, void* const* fld, const void* target,
+                  double ds, int32_t set_e, int32_t set_b, int32_t nfilter, void* stream);
+}  // namespace pic_internal
+
 namespace {
 
 template <typename real>
@@ -29,14 +35,8 @@ int gr_step(pic_ctx* ctx, const pic_gr_metric* m, pic_species* sp, int32_t nsp, 
   // +x2), match (+x1)
   const bool match  = gp.match_ds > 0.0;
   auto       bc_main = [&](int set_e, int set_b) {
-    for (int k = 0; k < 2; ++k) {
-      int s = pic_gr_field_bcs(ctx, m, f[k], set_e, set_b, p.nfilter, stream);
-      if (s == PIC_OK && match)
-        s = pic_gr_match_fields(ctx, m, f[k], gp.match_target, gp.match_ds, set_e, set_b,
-                                stream);
-      if (s != PIC_OK) return s;
-    }
-    return (int)PIC_OK;
+    return pic_internal::gr_boundaries(ctx, m, f, gp.match_target, match ? gp.match_ds : 0.0, set_e,
+                                       set_b, p.nfilter, stream);
   };
   auto swap = [&]() {
     std::swap(f[0], f[1]);
