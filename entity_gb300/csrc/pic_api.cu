@@ -270,6 +270,7 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
   a.st.rec    = c->stage_rec;
   a.st.claim  = c->stage_claim;
   a.st.nslots = c->stage_slots;
+  a.st.per_sm = std::max(1, c->stage_slots / pic::sm_count());
   e           = cudaErrorInvalidValue;
 #define PIC_TD(DD, OO) \
   if (D == DD && O == OO) e = pic::launch_push_deposit_tiled<DD, OO, real>(a, s);

@@ -134,12 +134,40 @@ struct TiledSpecies {
 // independent of the order of the additions. A full class hands its records
 // to the next one, which costs a bank conflict; the rows of a region hold a
 // whole chunk, so a record always finds a place. A CTA claims one of nslots
-// buffers; there are as many as CTAs that can be resident at once.
+// buffers; there are as many as CTAs that can be resident at once. A buffer
+// passes from one CTA to the next by a release and an acquire (take_slot,
+// give_slot): the last holder's records and discards come before the next
+// one's records.
 struct DepStage {
   uint4*    rec    = nullptr;  // nslots buffers of two regions (unmoved, moved)
   unsigned* claim  = nullptr;  // nslots words: 0 free, 1 held
-  int       nslots = 0;
+  int       nslots = 0, per_sm = 1;  // buffers, and CTAs resident on one SM
 };
+
+// Called by one thread. A buffer's index, or -1 when the limit ran out. The
+// search starts with this SM's own buffers, one of which its last CTA has just
+// given back. The fence orders the claim before the CTA's records (its other
+// warps start them behind a barrier).
+__device__ __forceinline__ int take_slot(const DepStage& st) {
+  const unsigned n = (unsigned)st.nslots;
+  unsigned       sm;
+  asm("mov.u32 %0, %%smid;" : "=r"(sm));
+  unsigned sl = (sm * (unsigned)st.per_sm) % n;
+  for (unsigned k = 0; k < 64u * n; ++k) {
+    if (atomicCAS(st.claim + sl, 0u, 1u) == 0u) {
+      __threadfence();
+      return (int)sl;
+    }
+    if (++sl == n) sl = 0;
+  }
+  return -1;
+}
+// Called by one thread behind a barrier that follows the CTA's last use of the
+// buffer: the fence orders every warp's records and discards before the word.
+__device__ __forceinline__ void give_slot(const DepStage& st, int slot) {
+  __threadfence();
+  atomicExch(st.claim + slot, 0u);
+}
 
 // drops the 128-byte line at p (128-byte aligned) from L2 without writing it
 // back; its contents are undefined until written again
@@ -360,24 +388,7 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
   }
   if (threadIdx.x == 0) {
     s_qmax = 0u;
-    s_slot = -1;
-    if constexpr (REC) {
-      // nslots is a multiple of the SMs: the search starts with this SM's own
-      // buffers, one of which its last CTA has just given back. The limit
-      // bounds the search all the same.
-      unsigned sm, nsm;
-      asm("mov.u32 %0, %%smid;" : "=r"(sm));
-      asm("mov.u32 %0, %%nsmid;" : "=r"(nsm));
-      const unsigned n = (unsigned)a.st.nslots, per = max(1u, n / max(1u, nsm));
-      unsigned       sl = (sm * per) % n;
-      for (unsigned k = 0; k < 64u * n; ++k) {
-        if (atomicCAS(a.st.claim + sl, 0u, 1u) == 0u) {
-          s_slot = (int)sl;
-          break;
-        }
-        if (++sl == n) sl = 0;
-      }
-    }
+    s_slot = REC ? take_slot(a.st) : -1;
   }
   __syncthreads();
   // (with the exact global accumulator the bound is the call's, known already)
@@ -417,7 +428,7 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
     if (__syncthreads_or(!done)) {
       if (threadIdx.x == 0) {
         atomicAdd(a.err + ERR_WAIT_TIMEOUT, 1ull);
-        if (REC && s_slot >= 0) atomicExch(a.st.claim + s_slot, 0u);
+        if (REC && s_slot >= 0) give_slot(a.st, s_slot);
       }
       return;
     }
@@ -675,7 +686,7 @@ __global__ void __launch_bounds__(TileShape<D, real, O>::NT, TileShape<D, real, 
     __syncthreads();
   }
   if constexpr (REC) {
-    if (threadIdx.x == 0) atomicExch(a.st.claim + s_slot, 0u);
+    if (threadIdx.x == 0) give_slot(a.st, s_slot);
   }
 
   // 3. flush the J window (periodic images folded onto active cells)
