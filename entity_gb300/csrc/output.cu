@@ -90,6 +90,13 @@ __device__ __forceinline__ real spline(real x) {
   return ZERO;
 }
 
+dim3 blocks_for(int64_t n) {
+  int64_t b = (n + 255) / 256;
+  if (b < 1) b = 1;
+  if (b > pic::sm_count() * 32) b = pic::sm_count() * 32;
+  return dim3((unsigned)b);
+}
+
 template <typename real>
 struct MomArgs {
   SpeciesPtrs     sp;
@@ -148,7 +155,7 @@ __device__ __forceinline__ bool moment_of(const MomArgs<real>& a, int64_t p, int
   return true;
 }
 
-// particles of a block, and its shared window
+// particles of a block of the windowed kernel, and its shared window
 constexpr int   kMomThreads = 512;
 constexpr float kMomSpread  = 32.f;  // largest coefficient over the mean one
 constexpr float kMomWeights = 64.f;  // largest weight over the smallest
@@ -157,11 +164,11 @@ constexpr int kMomWords   = 8 * 1024;  // 32 KB: 4096 nodes
 
 // a chunk's particles waiting for their deposit, queued by the shared-memory
 // bank (of 32) of their window's first node: row r holds the r-th of each bank
-template <int D, typename real>
+template <int D>
 struct MomQueue {
   int   word[kMomChunk];
   float dx[D][kMomChunk];
-  real  coeff[kMomChunk];
+  float coeff[kMomChunk];
 };
 // shape factors of one particle along each axis, and the products over its nodes
 template <int D, int ORDER, typename real>
@@ -206,36 +213,56 @@ __device__ __forceinline__ void moment_on_grid(const MomArgs<real>& a, const int
   });
 }
 
-template <int D, typename real>
-constexpr size_t moment_smem() {
-  return 4 * kMomWords + sizeof(MomQueue<D, real>);
+// ParticleMoments_kernel::operator() (particle_moments.hpp:291-404),
+// Cartesian, every particle's additions straight onto the grid
+template <int D, int ORDER, typename real>
+__global__ void __launch_bounds__(256) k_output_moment_direct(MomArgs<real> a,
+                                                              unsigned long long* err) {
+  const float*  da[3]  = { a.sp.dx1, a.sp.dx2, a.sp.dx3 };
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.sp.npart; p += stride) {
+    int   cell[3] = { 0, 0, 0 };
+    real  coeff, w;
+    bool  oob;
+    const bool ok = moment_of<D, real>(a, p, cell, coeff, w, oob);
+    if (oob) atomicAdd(err + ERR_OUT_OF_GRID, 1ull);
+    if (!ok) continue;
+    float dx[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) dx[d] = da[d][p];
+    moment_on_grid<D, ORDER, real>(a, cell, dx, coeff);
+  }
 }
 
-// ParticleMoments_kernel::operator() (particle_moments.hpp:291-404),
-// Cartesian. A block deposits kMomChunk consecutive particles. In FP32, where
-// these lie together (any spatial order: a box of cells that the window
+template <int D>
+constexpr size_t moment_smem() {
+  return 4 * kMomWords + sizeof(MomQueue<D>);
+}
+
+// The same in FP32 for many particles. A block deposits kMomChunk consecutive
+// ones. Where these lie together (any spatial order: a box of cells that the window
 // holds), it sums them in a shared-memory window in fixed point, scaled by the
 // block's largest coefficient, and adds the window's nodes to the grid once;
 // particles apart from the others (across a periodic edge, after a drift) add
 // to the grid directly, and so does a whole block in random order. Where the
 // block's coefficients do not suit the scale (not finite, too small, or so
 // unequal (kMomSpread, kMomWeights) that 30 bits below the largest would tell
-// in cells that hold small ones only) the window sums in double. FP64 adds to the grid directly: the fixed point
-// would be coarser than double.
+// in cells that hold small ones only) the window sums in double.
 // A particle makes (2 W + 1)^D additions, which bound the kernel. 16.8 M
 // sorted particles at order 2 took 1.64 ms with global atomics, which meet in
 // a few L2 lines, 1.05 ms in the window in their own order (the lanes of one
 // cell meet in its words, eight wavefronts an atomic), and 0.45 ms queued by
 // bank, a warp's 32 lanes adding in 32 banks.
-template <int D, int ORDER, typename real>
-__global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<real> a,
+template <int D, int ORDER>
+__global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<float> a,
                                                                unsigned long long* err) {
+  using real          = float;
   using FA            = FixedAcc<real>;
   constexpr int W     = (ORDER + 1) / 2;
   constexpr int NODES = kMomWords / FA::WORDS;
   constexpr int ROWS  = kMomChunk / 32;
   extern __shared__ __align__(16) unsigned win[];
-  MomQueue<D, real>& qu = *reinterpret_cast<MomQueue<D, real>*>(win + kMomWords);
+  MomQueue<D>& qu = *reinterpret_cast<MomQueue<D>*>(win + kMomWords);
   __shared__ int      s_lo[3], s_hi[3], s_mid[3], s_bad;
   __shared__ unsigned s_max, s_wlo, s_whi, s_cnt[32];
   __shared__ float    s_sum;
@@ -281,7 +308,7 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<real> a,
   // 2. the window: all cells, or those within 12 of the middle particle's
   int  w0[3] = { 0, 0, 0 }, wn[3] = { 1, 1, 1 };
   bool windowed = false;
-  if (sizeof(real) == 4 && s_lo[0] <= s_hi[0]) {
+  if (s_lo[0] <= s_hi[0]) {
     for (int t = 0; t < 2 && !windowed; ++t) {
       int64_t vol = 1;
 #pragma unroll
@@ -405,12 +432,20 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<real> a,
 
 template <int D, int ORDER, typename real>
 cudaError_t launch_moment(const MomArgs<real>& a, unsigned long long* err, cudaStream_t s) {
-  const size_t      smem = moment_smem<D, real>();
-  const unsigned    grid = (unsigned)((a.sp.npart + kMomChunk - 1) / kMomChunk);
-  const cudaError_t e    = cudaFuncSetAttribute(k_output_moment<D, ORDER, real>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  PIC_KL(k_output_moment<D, ORDER, real><<<grid, kMomThreads, smem, s>>>(a, err));
+  // FP64 adds to the grid: the window's fixed point would be coarser than double.
+  // In the windowed kernel, whose 128 KB of shared memory it asked for all the
+  // same, a 3D block of 512 threads had an SM to itself: 27,648 particles at order 2
+  // took 157 us there, 13 us so, 7.1 M 1.96 and 1.81 ms, 480,000 in 2D 88 and 68 us
+  if constexpr (sizeof(real) == 4) {
+    constexpr size_t  smem = moment_smem<D>();
+    const cudaError_t e    = cudaFuncSetAttribute(k_output_moment<D, ORDER>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    PIC_KL(k_output_moment<D, ORDER>
+           <<<(unsigned)((a.sp.npart + kMomChunk - 1) / kMomChunk), kMomThreads, smem, s>>>(a, err));
+  } else {
+    PIC_KL(k_output_moment_direct<D, ORDER, real><<<blocks_for(a.sp.npart), 256, 0, s>>>(a, err));
+  }
   return cudaGetLastError();
 }
 
@@ -537,13 +572,6 @@ __global__ void k_output_particles(PrtlOutArgs<real> a) {
     for (int d = 0; d < 3; ++d) a.u[d][p] = ux[d][q];
     a.w[p] = ((const real*)a.sp.w)[q];
   }
-}
-
-dim3 blocks_for(int64_t n) {
-  int64_t b = (n + 255) / 256;
-  if (b < 1) b = 1;
-  if (b > pic::sm_count() * 32) b = pic::sm_count() * 32;
-  return dim3((unsigned)b);
 }
 
 template <typename real>
