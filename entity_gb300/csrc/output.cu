@@ -21,7 +21,6 @@
 #include <cmath>
 
 #include "ctx_internal.cuh"
-#include "fixed_acc.cuh"
 
 using namespace pic_internal;
 
@@ -110,7 +109,7 @@ struct MomArgs {
 // Cartesian); false for one that is not deposited
 template <int D, typename real>
 __device__ __forceinline__ bool moment_of(const MomArgs<real>& a, int64_t p, int* cell, real& coeff,
-                                          real& w, bool& out_of_grid) {
+                                          bool& out_of_grid) {
   const real     ONE   = 1;
   const int32_t* ia[3] = { a.sp.i1, a.sp.i2, a.sp.i3 };
   const real*    ux[3] = { (const real*)a.sp.ux1, (const real*)a.sp.ux2, (const real*)a.sp.ux3 };
@@ -118,7 +117,7 @@ __device__ __forceinline__ bool moment_of(const MomArgs<real>& a, int64_t p, int
   const bool moving = a.id == PIC_MOM_T || a.id == PIC_MOM_V;
   const short tag   = a.sp.tag[p];
   real        u[3]  = { 0, 0, 0 };
-  w                 = a.use_weights ? ((const real*)a.sp.w)[p] : ONE;
+  const real  w     = a.use_weights ? ((const real*)a.sp.w)[p] : ONE;
   if (moving) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) u[c] = ux[c][p];
@@ -155,20 +154,48 @@ __device__ __forceinline__ bool moment_of(const MomArgs<real>& a, int64_t p, int
   return true;
 }
 
-// particles of a block of the windowed kernel, and its shared window
-constexpr int   kMomThreads = 512;
-constexpr float kMomSpread  = 32.f;  // largest coefficient over the mean one
-constexpr float kMomWeights = 64.f;  // largest weight over the smallest
-constexpr int kMomChunk   = 4096;
-constexpr int kMomWords   = 8 * 1024;  // 32 KB: 4096 nodes
+// The windowed kernel's block: threads, particles, nodes of its shared window
+template <int T, int C, int N>
+struct MomBlock {
+  static constexpr int THREADS = T, CHUNK = C, NODES = N;
+};
+using MomLarge = MomBlock<512, 4096, 4096>;
+
+// Window sums in fixed point. A contribution v, |v| <= 2^18, is split into
+// h + l 2^-19 (two words) or h + m 2^-19 + l 2^-38 (three), integers of at most 2^18
+// each, all but the last exact, and each is added to a 32-bit word: a chunk's additions
+// (2^12 at most) stay within 2^30. The integers come by adding 1.5 * 2^23, whose
+// sum's low mantissa bits they are.
+constexpr int kMomTop = 18, kMomStep = 19;
+template <int WORDS>
+__device__ __forceinline__ void moment_add(int* w, int plane, float v) {
+  const float MAGIC = 12582912.f, STEP = (float)(1 << kMomStep);
+  float       t = v + MAGIC, r = v - (t - MAGIC);
+  atomicAdd(w, __float_as_int(t) - 0x4B400000);
+#pragma unroll
+  for (int k = 1; k < WORDS; ++k) {
+    t = __fmaf_rn(r, STEP, MAGIC);
+    r = __fmaf_rn(r, STEP, MAGIC - t);
+    atomicAdd(w + k * plane, __float_as_int(t) - 0x4B400000);
+  }
+}
+// the sum of a node, in units of 2^-kMomStep
+template <int WORDS>
+__device__ __forceinline__ double moment_total(const int* w, int plane) {
+  const double t = (double)((long long)w[0] * (1 << kMomStep) + w[plane]);
+  return WORDS == 2 ? t : t + (double)w[(WORDS - 1) * plane] * (1.0 / (1 << kMomStep));
+}
+// the block's largest coefficient over the largest of a cell, at most, for two words
+// and for three
+constexpr float kMomRange2 = 256.f, kMomRange3 = 67108864.f;
 
 // a chunk's particles waiting for their deposit, queued by the shared-memory
 // bank (of 32) of their window's first node: row r holds the r-th of each bank
-template <int D>
+template <int D, typename B>
 struct MomQueue {
-  int   word[kMomChunk];
-  float dx[D][kMomChunk];
-  float coeff[kMomChunk];
+  int   word[B::CHUNK];
+  float dx[D][B::CHUNK];
+  float coeff[B::CHUNK];
 };
 // shape factors of one particle along each axis, and the products over its nodes
 template <int D, int ORDER, typename real>
@@ -222,9 +249,9 @@ __global__ void __launch_bounds__(256) k_output_moment_direct(MomArgs<real> a,
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < a.sp.npart; p += stride) {
     int   cell[3] = { 0, 0, 0 };
-    real  coeff, w;
+    real  coeff;
     bool  oob;
-    const bool ok = moment_of<D, real>(a, p, cell, coeff, w, oob);
+    const bool ok = moment_of<D, real>(a, p, cell, coeff, oob);
     if (oob) atomicAdd(err + ERR_OUT_OF_GRID, 1ull);
     if (!ok) continue;
     float dx[D];
@@ -234,39 +261,39 @@ __global__ void __launch_bounds__(256) k_output_moment_direct(MomArgs<real> a,
   }
 }
 
-template <int D>
+template <int D, typename B>
 constexpr size_t moment_smem() {
-  return 4 * kMomWords + sizeof(MomQueue<D>);
+  return 8 * B::NODES + sizeof(MomQueue<D, B>);
 }
 
-// The same in FP32 for many particles. A block deposits kMomChunk consecutive
-// ones. Where these lie together (any spatial order: a box of cells that the window
+// The same in FP32, a block depositing CHUNK consecutive particles. Where these
+// lie together (any spatial order: a box of cells that the window
 // holds), it sums them in a shared-memory window in fixed point, scaled by the
 // block's largest coefficient, and adds the window's nodes to the grid once;
 // particles apart from the others (across a periodic edge, after a drift) add
-// to the grid directly, and so does a whole block in random order. Where the
-// block's coefficients do not suit the scale (not finite, too small, or so
-// unequal (kMomSpread, kMomWeights) that 30 bits below the largest would tell
-// in cells that hold small ones only) the window sums in double.
+// to the grid directly, and so does a whole block in random order. The sums
+// have two words a node, 37 bits below the scale, where every occupied cell's largest
+// coefficient is within kMomRange2 of the block's, and three, 56 bits, where it is
+// within kMomRange3 (a cold region beside a hot one): an addition errs by 2^-29
+// of its cell's largest coefficient at most, where a float sum errs by 2^-24 of itself.
+// A block that neither suits (or whose coefficients are not finite, or too small) adds
+// to the grid, like one whose window has no room for the third word.
 // A particle makes (2 W + 1)^D additions, which bound the kernel. 16.8 M
 // sorted particles at order 2 took 1.64 ms with global atomics, which meet in
 // a few L2 lines, 1.05 ms in the window in their own order (the lanes of one
 // cell meet in its words, eight wavefronts an atomic), and 0.45 ms queued by
 // bank, a warp's 32 lanes adding in 32 banks.
-template <int D, int ORDER>
-__global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<float> a,
-                                                               unsigned long long* err) {
-  using real          = float;
-  using FA            = FixedAcc<real>;
-  constexpr int W     = (ORDER + 1) / 2;
-  constexpr int NODES = kMomWords / FA::WORDS;
-  constexpr int ROWS  = kMomChunk / 32;
-  extern __shared__ __align__(16) unsigned win[];
-  MomQueue<D>& qu = *reinterpret_cast<MomQueue<D>*>(win + kMomWords);
+template <int D, int ORDER, typename B>
+__global__ void __launch_bounds__(B::THREADS) k_output_moment(MomArgs<float> a,
+                                                              unsigned long long* err) {
+  using real         = float;
+  constexpr int W    = (ORDER + 1) / 2;
+  constexpr int ROWS = B::CHUNK / 32;
+  constexpr int kMomThreads = B::THREADS, kMomChunk = B::CHUNK;
+  extern __shared__ __align__(16) int win[];
+  MomQueue<D, B>& qu = *reinterpret_cast<MomQueue<D, B>*>(win + 2 * B::NODES);
   __shared__ int      s_lo[3], s_hi[3], s_mid[3], s_bad;
-  __shared__ unsigned s_max, s_wlo, s_whi, s_cnt[32];
-  __shared__ float    s_sum;
-  __shared__ int      s_num;
+  __shared__ unsigned s_max, s_min, s_cnt[32];
   const int32_t* ia[3] = { a.sp.i1, a.sp.i2, a.sp.i3 };
   const float*   da[3] = { a.sp.dx1, a.sp.dx2, a.sp.dx3 };
   const int64_t  p0    = (int64_t)blockIdx.x * kMomChunk;
@@ -274,7 +301,7 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<float> a,
   const int      tid = threadIdx.x, lane = tid & 31;
   if (tid < 3) s_lo[tid] = INT_MAX, s_hi[tid] = INT_MIN, s_mid[tid] = 0;
   if (tid < 32) s_cnt[tid] = 0u;
-  if (tid == 0) s_bad = 0, s_max = s_whi = 0u, s_wlo = ~0u, s_sum = 0.f, s_num = 0;
+  if (tid == 0) s_bad = 0, s_max = 0u, s_min = ~0u;
   __syncthreads();
   // 1. the block's box of cells (of all that lie in the grid)
   {
@@ -318,23 +345,22 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<float> a,
         w0[d] = lo - W, wn[d] = hi - lo + 1 + 2 * W;
         vol *= max(wn[d], 0);
       }
-      windowed = vol > 0 && vol <= NODES;
+      windowed = vol > 0 && vol <= B::NODES;
     }
   }
   const int nodes = wn[0] * wn[1] * wn[2];
   if (windowed)
-    for (int e = tid; e < nodes * FA::WORDS; e += kMomThreads) win[e] = 0u;
+    for (int e = tid; e < min(3 * nodes, 2 * B::NODES); e += kMomThreads) win[e] = 0;
+  __syncthreads();
   // 3. the window's particles into the queue, the others onto the grid
-  float    cmax = 0.f, csum = 0.f;
-  unsigned wlo = ~0u, whi = 0u;
-  int      num = 0;
-  bool     bad = false;
+  float cmax = 0.f;
+  bool  bad  = false;
 #pragma unroll 1
   for (int l = tid; l < n; l += kMomThreads) {
     int   cell[3] = { 0, 0, 0 };
-    real  coeff, w;
+    real  coeff;
     bool  oob;
-    const bool ok = moment_of<D, real>(a, p0 + l, cell, coeff, w, oob);
+    const bool ok = moment_of<D, real>(a, p0 + l, cell, coeff, oob);
     if (oob) atomicAdd(err + ERR_OUT_OF_GRID, 1ull);
     if (!ok) continue;
     float dx[D];
@@ -348,18 +374,14 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<float> a,
       moment_on_grid<D, ORDER, real>(a, cell, dx, coeff);
       continue;
     }
-    // beyond what the fixed-point scale covers
-    const float m = fabsf((float)coeff);
-    bad  = bad || !(m <= 0x1p126f) || (coeff != (real)0 && m < 0x1p-90f);
+    const float m = fabsf(coeff);
+    bad  = bad || !(m <= 0x1p126f);
     cmax = fmaxf(cmax, m);
-    csum += m;
-    ++num;
-    if (w != (real)0) {
-      wlo = min(wlo, __float_as_uint(fabsf((float)w)));
-      whi = max(whi, __float_as_uint(fabsf((float)w)));
-    }
     const int word = (cell[0] - W - w0[0]) +
                      wn[0] * ((cell[1] - W - w0[1]) + (D == 3 ? wn[1] * (cell[2] - W - w0[2]) : 0));
+    // the cell's largest coefficient, in the first word of its window's first
+    // node (non-negative floats order as their bits)
+    atomicMax(win + word, __float_as_int(m));
     // a full bank hands its particles to the next one; the queue holds them all
     unsigned cls = (unsigned)word, row = 0;
     for (int k = 0; k < 32; ++k, ++cls) {
@@ -375,59 +397,73 @@ __global__ void __launch_bounds__(kMomThreads) k_output_moment(MomArgs<float> a,
   }
   const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(cmax));
   if (!windowed) return;
-  wlo = __reduce_min_sync(0xffffffffu, wlo);
-  whi = __reduce_max_sync(0xffffffffu, whi);
-  num = __reduce_add_sync(0xffffffffu, num);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) csum += __shfl_xor_sync(0xffffffffu, csum, o);
-  if (lane == 0) {
-    atomicMax(&s_max, m);
-    atomicMin(&s_wlo, wlo), atomicMax(&s_whi, whi);
-    atomicAdd(&s_sum, csum), atomicAdd(&s_num, num);
-  }
+  if (lane == 0) atomicMax(&s_max, m);
   if (bad) s_bad = 1;
   __syncthreads();
-  const bool fixed = !s_bad && __uint_as_float(s_max) * (float)s_num <= kMomSpread * s_sum &&
-                     (s_whi == 0u || __uint_as_float(s_whi) <= kMomWeights * __uint_as_float(s_wlo));
+  // the least of the occupied cells' largest coefficients
+  unsigned least = ~0u;
+  for (int e = tid; e < nodes; e += kMomThreads) {
+    if (win[e] > 0) least = min(least, (unsigned)win[e]);
+    win[e] = 0;
+  }
+  least = __reduce_min_sync(0xffffffffu, least);
+  if (lane == 0) atomicMin(&s_min, least);
+  __syncthreads();
+  const float top = __uint_as_float(s_max), low = __uint_as_float(s_min);
+  if (top == 0.f) return;
+  const int words = s_bad || top < 0x1p-108f ? 0
+                    : top <= kMomRange2 * low ? 2
+                    : top <= kMomRange3 * low && 3 * nodes <= 2 * B::NODES ? 3 : 0;
   // 4. the queue into the window; |coefficient| < 2^ex, and its product with
   //    the shape factors stays below
-  int ex;
-  frexpf(__uint_as_float(s_max) * 1.0000002f, &ex);
-  const int  b     = FA::bits(kMomChunk);
-  const real scale = (real)ldexpf(1.f, b - ex), unscale = (real)ldexpf(1.f, ex - b);
-  const int  mine  = (int)min(s_cnt[lane], (unsigned)ROWS);
-  double*    sums  = reinterpret_cast<double*>(win);  // two words a node as well
-  for (int row = tid >> 5; row < mine; row += kMomThreads / 32) {
-    const int e = row * 32 + lane, word = qu.word[e];
-    float     dx[D];
+  int ex = 0;
+  if (words) frexpf(top * 1.0000002f, &ex);
+  const float scale = ldexpf(1.f, kMomTop - ex);
+  const int   mine  = (int)min(s_cnt[lane], (unsigned)ROWS);
+  auto deposit = [&](auto&& add) {
+    for (int row = tid >> 5; row < mine; row += kMomThreads / 32) {
+      const int e = row * 32 + lane, word = qu.word[e];
+      float     dx[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) dx[d] = qu.dx[d][e];
-    const MomShape<D, ORDER, real> S(dx, a.smoothing == PIC_SMOOTH_SPLINE);
-    const real                     coeff = qu.coeff[e], cs = coeff * scale;
-    if (fixed)
+      for (int d = 0; d < D; ++d) dx[d] = qu.dx[d][e];
+      const MomShape<D, ORDER, real> S(dx, a.smoothing == PIC_SMOOTH_SPLINE);
+      const real                     coeff = qu.coeff[e];
       S.each([&](int i, int j, int k, real sh) {
-        FA::add(win + word + i + wn[0] * (j + wn[1] * k), nodes, cs * sh);
+        add(word + i + wn[0] * (j + wn[1] * k), coeff, sh);
       });
-    else
-      S.each([&](int i, int j, int k, real sh) {
-        atomicAdd(sums + word + i + wn[0] * (j + wn[1] * k), (double)(coeff * sh));
-      });
-  }
-  __syncthreads();
-  for (int e = tid; e < nodes; e += kMomThreads) {
-    real v;
-    if (fixed) {
-      if (!FA::nonzero(win + e, nodes)) continue;
-      v = FA::to_real(FA::total(win + e, nodes), unscale);
-    } else {
-      v = (real)sums[e];
-      if (v == (real)0) continue;
     }
+  };
+  auto on_grid = [&](int e, real v) {
     const int i = e % wn[0], j = (e / wn[0]) % wn[1], k = e / (wn[0] * wn[1]);
     atomicAdd(a.buf.p + a.buf.idx(w0[0] + i + a.ng, w0[1] + j + a.ng, D == 3 ? w0[2] + k + a.ng : 0,
                                   a.comp),
               v);
+  };
+  if (words == 0) {
+    deposit([&](int e, real coeff, real sh) { on_grid(e, coeff * sh); });
+    return;
   }
+  if (words == 2)
+    deposit([&](int e, real coeff, real sh) { moment_add<2>(win + e, nodes, (coeff * scale) * sh); });
+  else
+    deposit([&](int e, real coeff, real sh) { moment_add<3>(win + e, nodes, (coeff * scale) * sh); });
+  __syncthreads();
+  const double unscale = ldexp(1.0, ex - kMomTop - kMomStep);
+  for (int e = tid; e < nodes; e += kMomThreads) {
+    const double v = words == 2 ? moment_total<2>(win + e, nodes) : moment_total<3>(win + e, nodes);
+    if (v != 0.0) on_grid(e, (real)(v * unscale));
+  }
+}
+
+template <int D, int ORDER, typename B>
+cudaError_t launch_moment_window(const MomArgs<float>& a, unsigned long long* err, cudaStream_t s) {
+  constexpr size_t  smem = moment_smem<D, B>();
+  const cudaError_t e    = cudaFuncSetAttribute(k_output_moment<D, ORDER, B>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  PIC_KL(k_output_moment<D, ORDER, B>
+         <<<(unsigned)((a.sp.npart + B::CHUNK - 1) / B::CHUNK), B::THREADS, smem, s>>>(a, err));
+  return cudaGetLastError();
 }
 
 template <int D, int ORDER, typename real>
@@ -437,16 +473,11 @@ cudaError_t launch_moment(const MomArgs<real>& a, unsigned long long* err, cudaS
   // same, a 3D block of 512 threads had an SM to itself: 27,648 particles at order 2
   // took 157 us there, 13 us so, 7.1 M 1.96 and 1.81 ms, 480,000 in 2D 88 and 68 us
   if constexpr (sizeof(real) == 4) {
-    constexpr size_t  smem = moment_smem<D>();
-    const cudaError_t e    = cudaFuncSetAttribute(k_output_moment<D, ORDER>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    PIC_KL(k_output_moment<D, ORDER>
-           <<<(unsigned)((a.sp.npart + kMomChunk - 1) / kMomChunk), kMomThreads, smem, s>>>(a, err));
+    return launch_moment_window<D, ORDER, MomLarge>(a, err, s);
   } else {
     PIC_KL(k_output_moment_direct<D, ORDER, real><<<blocks_for(a.sp.npart), 256, 0, s>>>(a, err));
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
 }
 
 // NormalizeVectorByRho_kernel (particle_moments.hpp:407-478): cmp::AlmostZero
