@@ -159,12 +159,13 @@ template <int T, int C, int N>
 struct MomBlock {
   static constexpr int THREADS = T, CHUNK = C, NODES = N;
 };
-using MomLarge = MomBlock<512, 4096, 4096>;
+using MomLarge = MomBlock<512, 2048, 4352>;
+using MomSmall = MomBlock<256, 512, 2560>;
 
 // Window sums in fixed point. A contribution v, |v| <= 2^18, is split into
 // h + l 2^-19 (two words) or h + m 2^-19 + l 2^-38 (three), integers of at most 2^18
 // each, all but the last exact, and each is added to a 32-bit word: a chunk's additions
-// (2^12 at most) stay within 2^30. The integers come by adding 1.5 * 2^23, whose
+// (2^11 at most) stay within 2^29. The integers come by adding 1.5 * 2^23, whose
 // sum's low mantissa bits they are.
 constexpr int kMomTop = 18, kMomStep = 19;
 template <int WORDS>
@@ -332,11 +333,24 @@ __global__ void __launch_bounds__(B::THREADS) k_output_moment(MomArgs<float> a,
     }
   }
   __syncthreads();
-  // 2. the window: all cells, or those within 12 of the middle particle's
+  // 2. the window: all cells, or those within 12 of the middle particle's where
+  //    these hold half of the particles
   int  w0[3] = { 0, 0, 0 }, wn[3] = { 1, 1, 1 };
   bool windowed = false;
   if (s_lo[0] <= s_hi[0]) {
     for (int t = 0; t < 2 && !windowed; ++t) {
+      if (t == 1) {
+        int near = 0;
+#pragma unroll
+        for (int k = 0; k < kMomChunk / kMomThreads; ++k) {
+          const int l  = k * kMomThreads + tid;
+          bool      in = l < n;
+#pragma unroll
+          for (int d = 0; d < D; ++d) in = in && abs(ia[d][p0 + l] - s_mid[d]) <= 12;
+          near += __syncthreads_count(in);
+        }
+        if (2 * near < n) break;
+      }
       int64_t vol = 1;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
@@ -473,7 +487,9 @@ cudaError_t launch_moment(const MomArgs<real>& a, unsigned long long* err, cudaS
   // same, a 3D block of 512 threads had an SM to itself: 27,648 particles at order 2
   // took 157 us there, 13 us so, 7.1 M 1.96 and 1.81 ms, 480,000 in 2D 88 and 68 us
   if constexpr (sizeof(real) == 4) {
-    return launch_moment_window<D, ORDER, MomLarge>(a, err, s);
+    return a.sp.npart / MomLarge::CHUNK >= 3 * pic::sm_count()
+             ? launch_moment_window<D, ORDER, MomLarge>(a, err, s)
+             : launch_moment_window<D, ORDER, MomSmall>(a, err, s);
   } else {
     PIC_KL(k_output_moment_direct<D, ORDER, real><<<blocks_for(a.sp.npart), 256, 0, s>>>(a, err));
     return cudaGetLastError();
