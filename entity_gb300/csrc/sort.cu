@@ -22,6 +22,7 @@
 // (128^3 cells, with the injection) went from 9.45 to 4.19 ms.
 // Nothing here synchronises with the host; the dead count stays on the
 // device until the caller reads it.
+#include <climits>
 #include <type_traits>
 
 #include <cuda_runtime.h>
@@ -362,18 +363,38 @@ __device__ __forceinline__ int32_t index_at(const SortArgs& a, int64_t p) {
 
 // bins above kBigBin: their indices put in order in a.rank (free after the
 // scatter) by rank counting (O(m^2 / threads)); blocks stride over the bins
-// the counting listed, whose number only the device knows
+// the counting listed, whose number only the device knows. The indices are counted
+// from shared memory, 1024 at a time: read from the records, which lie 64 bytes
+// apart, 12^3 bins of 1500 took a sort of 2.86 ms
+// (1.08 so; 1.75 with the indices in an array of their own).
 template <typename R>
-__global__ void k_fix_big(SortArgs a) {
-  const int nbig = *a.nbig;
+__global__ void __launch_bounds__(256) k_fix_big(SortArgs a) {
+  __shared__ int4 s_idx[256];
+  const int nbig = *a.nbig, tid = threadIdx.x;
   for (int bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
     const int     b  = a.big[bi];
     const int64_t lo = a.off[b], hi = a.off[b + 1];
-    for (int64_t q = lo + threadIdx.x; q < hi; q += blockDim.x) {
-      const int32_t x = index_at<R>(a, q);
+    for (int64_t q0 = lo; q0 < hi; q0 += 256) {
+      const int64_t q = q0 + tid;
+      const int32_t x = q < hi ? index_at<R>(a, q) : 0;
       int64_t       r = lo;
-      for (int64_t z = lo; z < hi; ++z) r += index_at<R>(a, z) < x;
-      a.rank[r] = x;
+      for (int64_t z0 = lo; z0 < hi; z0 += 1024) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int64_t z = z0 + k * 256 + tid;
+          reinterpret_cast<int32_t*>(s_idx)[k * 256 + tid] = z < hi ? index_at<R>(a, z) : INT_MAX;
+        }
+        __syncthreads();
+        int smaller = 0;
+#pragma unroll 4
+        for (int k = 0; k < 256; ++k) {
+          const int4 v = s_idx[k];
+          smaller += (v.x < x) + (v.y < x) + (v.z < x) + (v.w < x);
+        }
+        r += smaller;
+      }
+      if (q < hi) a.rank[r] = x;
     }
   }
 }
