@@ -374,7 +374,7 @@ __global__ void k_filter(GridInfo g, CellIter it, FieldView<real> src, FieldView
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
 #define b(x, y, z) src.p[src.idx(x, y, z, c)]
-      static_assert(D == 2, "the 3D pass is k_filter3_march");
+      static_assert(D == 2, "the 3D passes are below");
       nv[c] = INV_4 * b(i1, i2, 0) +
               INV_8 * (b(i1 - 1, i2, 0) + b(i1 + 1, i2, 0) + b(i1, i2 - 1, 0) + b(i1, i2 + 1, 0)) +
               INV_16 * (b(i1 - 1, i2 - 1, 0) + b(i1 + 1, i2 + 1, 0) + b(i1 - 1, i2 + 1, 0) +
@@ -393,7 +393,7 @@ __global__ void k_filter(GridInfo g, CellIter it, FieldView<real> src, FieldView
 // one component's 27-point sum, the terms in the reference's order
 // (digital_filter.hpp:352-379; the (i, j, k +- 1) pair appears twice in the 1/32
 // group, as in :365); b[z][y][x] is the cell's neighbourhood
-template <typename T, typename real>
+template <typename T>
 __device__ __forceinline__ T filter_sum(const T (*b)[3][3], T i8, T i16, T i32, T i64) {
 #define B(x, y, z) b[(z) + 1][(y) + 1][(x) + 1]
   return i8 * B(0, 0, 0) +
@@ -405,18 +405,18 @@ __device__ __forceinline__ T filter_sum(const T (*b)[3][3], T i8, T i16, T i32, 
 #undef B
 }
 
-// The 3D pass: a block of 32 x 8 threads marches along x3 over zlen cells, with
+// The 3D pass in FP32: a block of 32 x 8 threads marches along x3 over zlen cells, with
 // the plane ahead staged in shared memory (double-buffered, one-cell halo) and
 // each thread's last three 3 x 3 neighbourhoods of each component in
-// registers: a cell reads 9 new values per component, not 27. In FP32 the first
+// registers: a cell reads 9 new values per component, not 27. The first
 // two components are summed as one packed operation. The terms and their order
-// are the reference's: the same bits. 256^3 FP32: 307 us a pass with every cell
+// are the reference's: the same bits. 256^3: 307 us a pass with every cell
 // reading its 27 values from a staged block (665 instructions per cell), 220 us;
 // 100 x 75 x 61 18.6 and 14.5 us.
 constexpr int kFltX = 32, kFltY = 8;
-template <typename real>
-__global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<real> src,
-                                                       FieldView<real> dst, int zlen) {
+__global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<float> src,
+                                                       FieldView<float> dst, int zlen) {
+  using real = float;
   constexpr int SX = kFltX + 2, SY = kFltY + 2, PLANE = SX * SY, NS = 3 * PLANE,
                 TRIPS = (NS + 255) / 256;
   __shared__ real sm[2][NS];
@@ -431,9 +431,8 @@ __global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<rea
   const real* from[TRIPS];
 #pragma unroll
   for (int k = 0; k < TRIPS; ++k) {
-    const int t = threadIdx.x + k * 256, c = t / PLANE, y = (t % PLANE) / SX, x = t % SX;
+    const int t = threadIdx.x + k * 256, c = t / PLANE, y = (t % PLANE) / SX;
     const int gx = x0 - 1 + (t % PLANE) % SX, gy = y0 - 1 + y;
-    (void)x;
     from[k] = t < NS && gx < ex && gy < ey ? src.p + src.idx(gx, gy, 0, c) : nullptr;
   }
   real v[TRIPS];
@@ -451,9 +450,7 @@ __global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<rea
   const real  INV_8 = 0.125, INV_16 = 0.0625, INV_32 = 0.03125, INV_64 = 0.015625;
   const int   i1 = x0 + tx, i2 = y0 + ty;
   const bool  mine = i1 < g.n[0] + ng && i2 < g.n[1] + ng;
-  using Pair = std::conditional_t<sizeof(real) == 4, F2, real>;
-  Pair bp[3][3][3];                            // FP32: components 0 and 1; else component 0
-  real b1[sizeof(real) == 4 ? 1 : 3][3][3];    // FP64: component 1
+  F2   bp[3][3][3];  // components 0 and 1
   real b2[3][3][3];
   auto take = [&](int buf, int z) {  // plane z of the neighbourhoods from a buffer
 #pragma unroll
@@ -461,13 +458,8 @@ __global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<rea
 #pragma unroll
       for (int x = 0; x < 3; ++x) {
         const real* q = &sm[buf][(ty + y) * SX + tx + x];
-        if constexpr (sizeof(real) == 4) {
-          bp[z][y][x] = f2(q[0], q[PLANE]);
-        } else {
-          bp[z][y][x] = q[0];
-          b1[z][y][x] = q[PLANE];
-        }
-        b2[z][y][x] = q[2 * PLANE];
+        bp[z][y][x]   = f2(q[0], q[PLANE]);
+        b2[z][y][x]   = q[2 * PLANE];
       }
   };
   auto shift = [&]() {
@@ -479,7 +471,6 @@ __global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<rea
         for (int x = 0; x < 3; ++x) {
           bp[z][y][x] = bp[z + 1][y][x];
           b2[z][y][x] = b2[z + 1][y][x];
-          if constexpr (sizeof(real) == 8) b1[z][y][x] = b1[z + 1][y][x];
         }
   };
   fetch(z0 - 1);
@@ -499,16 +490,11 @@ __global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<rea
     shift();
     take(buf, 2);
     if (mine) {
-      real nv[3];
-      if constexpr (sizeof(real) == 4) {
-        const F2 r = filter_sum<F2, real>(bp, f2(INV_8, INV_8), f2(INV_16, INV_16),
-                                          f2(INV_32, INV_32), f2(INV_64, INV_64));
-        unpack(r, nv[0], nv[1]);
-      } else {
-        nv[0] = filter_sum<real, real>(bp, INV_8, INV_16, INV_32, INV_64);
-        nv[1] = filter_sum<real, real>(b1, INV_8, INV_16, INV_32, INV_64);
-      }
-      nv[2] = filter_sum<real, real>(b2, INV_8, INV_16, INV_32, INV_64);
+      real     nv[3];
+      const F2 r = filter_sum(bp, f2(INV_8, INV_8), f2(INV_16, INV_16), f2(INV_32, INV_32),
+                              f2(INV_64, INV_64));
+      unpack(r, nv[0], nv[1]);
+      nv[2] = filter_sum(b2, INV_8, INV_16, INV_32, INV_64);
 #pragma unroll
       for (int c = 0; c < 3; ++c) dst.p[dst.idx(i1, i2, i3, c)] = nv[c];
       for_images<3>(g, i1, i2, i3, [&](int a, int bb, int e) {
@@ -517,6 +503,69 @@ __global__ void __launch_bounds__(256) k_filter3_march(GridInfo g, FieldView<rea
       });
     }
   }
+}
+
+// The 3D pass in FP64: a block holds 32 x 8 cells of one plane and a one-cell halo of
+// the three components in shared memory, and each cell's sum reads its 27 values there.
+// The sums are bound by the FP64 pipe, two lanes per SM and clock, and want many warps:
+// marching with the neighbourhoods in registers took 65.6 us a pass at 64^3, 473 at
+// 128^3 and 1432 at 192^3, blocks of four planes 59.6, 381 and 1231, of one plane
+// 53.3, 367 and 1220 (24^3: 12.4, 34.9 and 12.4).
+__global__ void __launch_bounds__(256) k_filter3_staged(GridInfo g, FieldView<double> src,
+                                                        FieldView<double> dst) {
+  constexpr int SX = kFltX + 2, SY = kFltY + 2, SZ = 3, NS = 3 * SZ * SY * SX,
+                TRIPS = (NS + 255) / 256;
+  __shared__ double sm[3][SZ][SY][SX];
+  const int ng = g.ng;
+  // first active cell of the block, ghost-inclusive
+  const int x0 = ng + blockIdx.x * kFltX, y0 = ng + blockIdx.y * kFltY, i3 = ng + blockIdx.z;
+  const int ex = g.n[0] + 2 * ng, ey = g.n[1] + 2 * ng;
+  // a fixed trip count, unrolled: every thread's loads are in flight together
+  double v[TRIPS];
+#pragma unroll
+  for (int k = 0; k < TRIPS; ++k) {
+    const int t = threadIdx.x + k * 256;
+    const int x = t % SX, y = (t / SX) % SY, z = (t / (SX * SY)) % SZ, c = t / (SX * SY * SZ);
+    const int gx = x0 - 1 + x, gy = y0 - 1 + y, gz = i3 - 1 + z;
+    // cells past the array belong to no active cell of this block
+    v[k] = t < NS && gx < ex && gy < ey ? src.p[src.idx(gx, gy, gz, c)] : 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < TRIPS; ++k) {
+    const int t = threadIdx.x + k * 256;
+    if (t < NS) (&sm[0][0][0][0])[t] = v[k];
+  }
+  __syncthreads();
+  const int tx = threadIdx.x % kFltX, ty = threadIdx.x / kFltX;
+  const int i1 = x0 + tx, i2 = y0 + ty;
+  if (i1 >= g.n[0] + ng || i2 >= g.n[1] + ng) return;
+  double nv[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    double b[3][3][3];
+#pragma unroll
+    for (int q = 0; q < 27; ++q) b[q / 9][q / 3 % 3][q % 3] = sm[c][q / 9][ty + q / 3 % 3][tx + q % 3];
+    nv[c] = filter_sum(b, 0.125, 0.0625, 0.03125, 0.015625);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) dst.p[dst.idx(i1, i2, i3, c)] = nv[c];
+  for_images<3>(g, i1, i2, i3, [&](int a, int bb, int e) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) dst.p[dst.idx(a, bb, e, c)] = nv[c];
+  });
+}
+
+void filter3(const GridInfo& g, FieldView<float> a, FieldView<float> b, cudaStream_t s) {
+  // x3 cells per block: as many as leave four blocks per SM, 4 to 16 (a block
+  // stages two planes more than it has cells; 100 x 75 x 61: 14.5 us, 23.0 with 16)
+  const int     bx = (g.n[0] + kFltX - 1) / kFltX, by = (g.n[1] + kFltY - 1) / kFltY;
+  const int64_t fit  = (int64_t)bx * by * g.n[2] / (4 * pic::sm_count());
+  const int     zlen = (int)std::min<int64_t>(16, std::max<int64_t>(4, fit));
+  PIC_KL(k_filter3_march<<<dim3(bx, by, (g.n[2] + zlen - 1) / zlen), 256, 0, s>>>(g, a, b, zlen));
+}
+void filter3(const GridInfo& g, FieldView<double> a, FieldView<double> b, cudaStream_t s) {
+  const dim3 blocks((g.n[0] + kFltX - 1) / kFltX, (g.n[1] + kFltY - 1) / kFltY, g.n[2]);
+  PIC_KL(k_filter3_staged<<<blocks, 256, 0, s>>>(g, a, b));
 }
 
 // copy all cells (ghost-inclusive) of a 3-component field
@@ -676,21 +725,12 @@ cudaError_t launch_filter(const GridInfo& g, FieldView<real> J, FieldView<real> 
   const int64_t  ncells_g = (int64_t)(g.n[0] + 2 * g.ng) * (g.n[1] + 2 * g.ng) *
                            (g.dim == 3 ? g.n[2] + 2 * g.ng : 1) * 3;
   const dim3     grc      = grid_for(ncells_g, 256);
-  // x3 cells per block: as many as leave four blocks per SM, up to 16 (a block
-  // stages two planes more than it has cells); no fewer than 4 in FP32, where
-  // the staging is the cost (100 x 75 x 61: 14.5 us, 23.0 with 16), and down to
-  // 1 in FP64, bound by the FP64 pipe (64^3: 64.8 us, 65.4 with 4, 125 with 16)
-  const int bx = (g.n[0] + kFltX - 1) / kFltX, by = (g.n[1] + kFltY - 1) / kFltY;
-  const int nz   = g.dim == 3 ? g.n[2] : 1;
-  const int zlen = (int)std::min<int64_t>(
-    16, std::max<int64_t>(sizeof(real) == 4 ? 4 : 1, (int64_t)bx * by * nz / (4 * pic::sm_count())));
-  const dim3 gs(bx, by, (nz + zlen - 1) / zlen);
   if (all_per) {
     // ping-pong: every ghost cell is an image and is rewritten each pass
     FieldView<real> a = J, b = buff;
     for (int p = 0; p < npasses; ++p) {
       if (g.dim == 2) PIC_KL(k_filter<2, real><<<gr, 256, 0, s>>>(g, it, a, b));
-      else            PIC_KL(k_filter3_march<real><<<gs, 256, 0, s>>>(g, a, b, zlen));
+      else            filter3(g, a, b, s);
       FieldView<real> t = a;
       a                 = b;
       b                 = t;
@@ -701,7 +741,7 @@ cudaError_t launch_filter(const GridInfo& g, FieldView<real> J, FieldView<real> 
     for (int p = 0; p < npasses; ++p) {
       PIC_KL(k_copy3<real><<<grc, 256, 0, s>>>(g, J, buff));
       if (g.dim == 2) PIC_KL(k_filter<2, real><<<gr, 256, 0, s>>>(g, it, buff, J));
-      else            PIC_KL(k_filter3_march<real><<<gs, 256, 0, s>>>(g, buff, J, zlen));
+      else            filter3(g, buff, J, s);
     }
   }
   return cudaGetLastError();
