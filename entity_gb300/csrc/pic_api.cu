@@ -220,18 +220,19 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
   a.err        = c->d_err;
   const int D = c->grid.dim, O = c->grid.order;
   {
-    // 2D: the lanes of a warp spread over about four cells, the stride from the
-    // species' mean particles per cell (they deposit as they are pushed). 3D:
-    // consecutive particles (their deposit is ordered by its records, and the
-    // field reads of one cell broadcast). Strides 1, 2 and 4 took 13.4, 13.7
-    // and 14.3 ms per step of the 96^3 sweep plasma, 0.998, 1.040 and 1.108 ms
-    // of 100 x 75 x 61 turbulence, 0.447, 0.424 and 0.431 ms of the 512^2 pair
-    // plasma (16 ppc)
+    // Where particles deposit as they are pushed (2D, and order 0): the lanes of
+    // a warp spread over about four cells, the stride from the species' mean
+    // particles per cell. 3D at orders 1-3: consecutive particles (their deposit
+    // is ordered by its records, and the field reads of one cell broadcast).
+    // Strides 1, 2 and 4 took 13.4, 13.7 and 14.3 ms per step of the 96^3 sweep
+    // plasma, 0.998, 1.040 and 1.108 ms of 100 x 75 x 61 turbulence, 0.447, 0.424
+    // and 0.431 ms of the 512^2 pair plasma (16 ppc); at order 0 64^3 cells with
+    // 2 x 16 ppc took 864 us with stride 1, 574 us with 2
     int64_t np = 0, cells = 1;
     for (int k = 0; k < a.nsp; ++k) np += sps[k]->npart;
     for (int d = 0; d < D; ++d) cells *= c->grid.n[d];
     const int64_t ppc = np / std::max<int64_t>(1, (int64_t)a.nsp * cells);
-    a.lane_stride     = D == 3 || ppc < 12 ? 1 : (ppc >= 24 ? 4 : 2);
+    a.lane_stride     = (D == 3 && O >= 1) || ppc < 12 ? 1 : (ppc >= 24 ? 4 : 2);
   }
   cudaError_t e = cudaErrorInvalidValue;
   if (!c->stage_tried) {
