@@ -224,7 +224,9 @@ __global__ void __launch_bounds__(256, (D == 2 && sizeof(real) == 4)
 // one launch (blockIdx.y). The lists are short and a particle is one long chain
 // of latencies, so the lists share the SMs: two of 512^2 pairs took 9.5 us each
 // in launches of their own, 14 us together, two of 100 x 75 x 61 turbulence 25
-// and 45 us.
+// and 45 us. Order 3 in 3D asks for three blocks per SM: 2 x 2.1 M particles all in
+// the lists took 3.64 ms, with four 4.34 ms (order 2 1.42 and 1.45, order 1 0.63 and
+// 0.56).
 constexpr int kMaxTiledSpecies = 4;
 template <typename real>
 struct DrainArgs {
@@ -232,7 +234,7 @@ struct DrainArgs {
   int          n = 0;
 };
 template <int D, int O, typename real>
-__global__ void __launch_bounds__(128, (D == 2 && sizeof(real) == 4) ? 6 : 4)
+__global__ void __launch_bounds__(128, (D == 2 && sizeof(real) == 4) ? 6 : (O == 3 ? 3 : 4))
     k_push_deposit_lists(const __grid_constant__ DrainArgs<real> d) {
   push_deposit_all<D, O, real, MODE_FUSED, false, false>(d.s[blockIdx.y]);
 }
