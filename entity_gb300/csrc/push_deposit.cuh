@@ -127,7 +127,10 @@ __device__ __forceinline__ void fixed_scale(const FixedJ& fj, float& scale, int&
 
 // 2D FP32 asks for three CTAs per SM (80 registers instead of the
 // allocator's 96, an 8-byte spill): the never-sorted two-stream adjoint
-// problem's forward, which runs here, went from 134.1 to 128.8 ms
+// problem's forward, which runs here, went from 134.1 to 128.8 ms. 3D FP32 at order
+// 3 asks for two (128 registers of 255) where it pushes: 3.5 M particles in random
+// order 5.20 and 4.54 ms fused, 2.46 and 2.21 ms pushed, in cell order 3.32 and 2.80,
+// 1.08 and 0.84 ms.
 // VEC (FP32): the fields are read by rows (VecField), and float currents added
 // by rows (red_row). Particles in random order are bound by the lines and atomics
 // of their stencils in L1 and L2, rows are two thirds fewer: 14.2 M particles at
@@ -215,7 +218,8 @@ __device__ __forceinline__ void push_deposit_all(const PDArgs<real>& a) {
 template <int D, int O, typename real, int MODE, bool PHOTON, bool VEC>
 __global__ void __launch_bounds__(256, (D == 2 && sizeof(real) == 4)
                                            ? 3
-                                           : (VEC ? (MODE == MODE_DEPOSIT ? 3 : 2) : 1))
+                                           : (VEC ? (MODE == MODE_DEPOSIT ? 3 : 2)
+                                                  : (O == 3 && sizeof(real) == 4 && MODE != MODE_DEPOSIT ? 2 : 1)))
     k_push_deposit(const __grid_constant__ PDArgs<real> a) {
   push_deposit_all<D, O, real, MODE, PHOTON, VEC>(a);
 }
