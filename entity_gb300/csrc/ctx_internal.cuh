@@ -60,7 +60,8 @@ struct pic_ctx {
   // SR field boundaries (pic_set_field_bcs)
   pic_field_bcs                                   fbc = {};
   // exact current accumulator of pic_push_deposit (FP32; grown on demand):
-  // 3 x the ghost-inclusive cells of 64-bit totals, and the call's bound
+  // 3 x the ghost-inclusive cells of 64-bit totals, and two words: the call's bound, and
+  // which kernel takes a species (PDArgs::chunked)
   long long*                                      jfix       = nullptr;
   size_t                                          jfix_elems = 0;
   unsigned*                                       jfix_bound = nullptr;

@@ -6,10 +6,60 @@
 
 namespace pic {
 
+// One block of 256 threads looks at every fourth particle of 32 chunks over a species:
+// whether the cells of three chunks in four fit a window. All its loads are in flight
+// together (one after another they took 25 us).
+__device__ __forceinline__ void chunk_order(const BoundArgs& a, int s) {
+  constexpr int EACH   = 4;  // chunks of a warp, and particles of a lane in each
+  const int     lane   = threadIdx.x & 31;
+  const int64_t chunks = (a.n[s] + kChunk - 1) / kChunk, part = chunks / 32 + 1;
+  static_assert(kChunk == 32 * EACH * 4, "a fourth of a chunk");
+  int c[EACH][EACH][2];
+#pragma unroll
+  for (int r = 0; r < EACH; ++r) {
+    // at another place in each thirty-second: equal steps can meet a row's end each time
+    const int     w  = (threadIdx.x >> 5) * EACH + r;
+    const int64_t p0 = (chunks * w / 32 + w * 29 % part) % chunks * kChunk;
+#pragma unroll
+    for (int k = 0; k < EACH; ++k) {
+      int64_t p = p0 + (k * 32 + lane) * 4;
+      p         = p < a.n[s] ? p : a.n[s] - 1;
+#pragma unroll
+      for (int d = 0; d < 2; ++d) c[r][k][d] = a.cells[s][d][p];
+    }
+  }
+  int fit = 0;
+#pragma unroll
+  for (int r = 0; r < EACH; ++r) {
+    int64_t nodes = 1;
+    bool    some  = true;
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      int lo = INT_MAX, hi = INT_MIN;
+#pragma unroll
+      for (int k = 0; k < EACH; ++k)
+        if (cells_in_grid<2>(c[r][k], a.grid)) lo = min(lo, c[r][k][d]), hi = max(hi, c[r][k][d]);
+      lo   = __reduce_min_sync(0xffffffffu, lo);
+      hi   = __reduce_max_sync(0xffffffffu, hi);
+      some = some && lo <= hi;
+      nodes *= (int64_t)hi - lo + 6;
+    }
+    fit += some && nodes <= kChunkNodes;
+  }
+  __shared__ int s_fit;
+  if (threadIdx.x == 0) s_fit = 0;
+  __syncthreads();
+  if (lane == 0) atomicAdd(&s_fit, fit);
+  __syncthreads();
+  if (threadIdx.x == 0) *a.chunked[s] = 4 * s_fit >= 3 * 32;
+}
+
 // max |w| |q| over the weights of up to kBoundSpecies species (blockIdx.y);
-// 16-byte loads where the array allows, one atomic per block
-__global__ void k_weight_bound(BoundArgs a) {
+// 16-byte loads where the array allows, one atomic per block. A species whose order is
+// asked for has its first block do that besides.
+__global__ void k_weight_bound(const __grid_constant__ BoundArgs a) {
   const int     s      = blockIdx.y;
+  if (blockIdx.x == 0 && a.chunked[s]) chunk_order(a, s);
   const float*  w      = a.w[s];
   const int64_t n      = a.n[s];
   const int64_t tid    = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -53,7 +53,16 @@ struct BoundArgs {
   float        q[kBoundSpecies];  // |charge|
   int          ns = 0;
   unsigned*    bound = nullptr;
+  // 2D species whose order is asked for as well (chunked[s] not null): set to 1 where
+  // k_push_deposit_chunk takes the particles, to 0 where the per-particle kernel does
+  const int32_t* cells[kBoundSpecies][2] = {};
+  unsigned*      chunked[kBoundSpecies]  = {};
+  int            grid[2] = { 0, 0 };  // cells of the grid
 };
+// k_push_deposit_chunk: particles of a block, and the nodes its window holds (48
+// bytes each: 38 KB, four blocks per SM)
+constexpr int kChunk      = 512;
+constexpr int kChunkNodes = 800;
 cudaError_t launch_weight_bound(const BoundArgs& a, cudaStream_t s);
 
 // J (+)= the totals in real_t: every element written when overwrite, else

@@ -103,7 +103,7 @@ cudaError_t pd_dispatch(const pic_ctx* c, const pic::PDArgs<real>& a, int mode, 
 template <typename real>
 int run_pd(pic_ctx* c, const pic_species* sp, const void* EB, void* J, double dt, double omegaB0,
            double dx, int mode, bool write_prev, cudaStream_t s,
-           const pic::FixedJ* fj = nullptr) {
+           const pic::FixedJ* fj = nullptr, const unsigned* chunked = nullptr) {
   pic::PDArgs<real> a;
   if (fj) a.fj = *fj;
   a.sp = sptrs(sp);
@@ -129,6 +129,7 @@ int run_pd(pic_ctx* c, const pic_species* sp, const void* EB, void* J, double dt
   a.vay              = sp->pusher == PIC_PUSHER_VAY;
   a.write_prev       = write_prev ? 1 : 0;
   a.err              = c->d_err;
+  a.chunked          = chunked;
   return cuda_status(pd_dispatch<real>(c, a, mode, photon, s));
 }
 
@@ -622,6 +623,20 @@ int pic_deposit(pic_ctx* c, const pic_species* sp, int32_t nspecies, void* J, do
   return PIC_OK;
 }
 
+// Where the windows of k_push_deposit_chunk can pay for an unbinned species in cell
+// order, which the device finds out; us per call by particles and in windows, cell
+// order, 256^2: order 2 with 8, 16 and 32 per cell 92/65, 156/103 and 292/169, order 3
+// 158/92, 297/157 and 588/260, order 1 51/46, 82/71 and 138/110. Order 1, few
+// particles and few per cell go without: the kernel that leaves at once and the look at
+// the order take 5 us. In random order windows lose (900^2, 32 per cell, order 2: 5.8
+// ms instead of 4.5).
+static bool windows_may_pay(const pic_ctx* c, const pic_species& sp) {
+  return c->grid.dim == 2 && c->grid.order >= 2 && sp.pusher != PIC_PUSHER_PHOTON &&
+         sp.npart >= (1 << 19) && sp.npart >= 8 * (int64_t)c->grid.n[0] * c->grid.n[1];
+}
+// words for the first species of a call (pic::BoundArgs::chunked)
+static constexpr int kOrderWords = 16;
+
 // Arms the exact current accumulator for one FP32 pic_push_deposit call over
 // the species that deposit: clears the totals and the bound, then bounds
 // |q w| over their particles. Returns false when the accumulator cannot be
@@ -643,7 +658,7 @@ bool arm_fixed_J(pic_ctx* c, const pic_species* sp, int32_t nspecies, double dt,
     }
     c->jfix_elems = elems;
   }
-  if (!c->jfix_bound && cudaMalloc((void**)&c->jfix_bound, sizeof(unsigned)) != cudaSuccess) {
+  if (!c->jfix_bound && cudaMalloc((void**)&c->jfix_bound, (1 + kOrderWords) * sizeof(unsigned)) != cudaSuccess) {
     cudaGetLastError();
     c->jfix_bound = nullptr;
     return false;
@@ -653,12 +668,18 @@ bool arm_fixed_J(pic_ctx* c, const pic_species* sp, int32_t nspecies, double dt,
     return false;
   int64_t         ntot = 0;
   pic::BoundArgs  ba;
-  ba.bound = c->jfix_bound;
+  ba.bound   = c->jfix_bound;
+  ba.grid[0] = c->grid.n[0];
+  ba.grid[1] = c->grid.n[1];
   for (int k = 0; k < nspecies; ++k) {
     const pic_species* q = sp + k;
     if (q->pusher == PIC_PUSHER_NONE || q->npart == 0 || q->charge == 0.0f) continue;
     ntot += q->npart;
     ba.w[ba.ns] = (const float*)q->weight;
+    const bool ask     = k < kOrderWords && windows_may_pay(c, *q);
+    ba.cells[ba.ns][0] = q->i1;
+    ba.cells[ba.ns][1] = q->i2;
+    ba.chunked[ba.ns]  = ask ? c->jfix_bound + 1 + k : nullptr;
     ba.n[ba.ns] = q->npart;
     ba.q[ba.ns] = std::fabs(q->charge);
     if (++ba.ns == pic::kBoundSpecies) {
@@ -703,7 +724,11 @@ int pic_push_deposit(pic_ctx* c, const pic_species* sp, int32_t nspecies, const 
   // kernel together; the rest, and any particles beyond a binned prefix,
   // through the per-particle kernel
   std::vector<const pic_species*> tiled;
-  std::vector<pic_species>        rest;
+  struct Rest {
+    pic_species     sp;
+    const unsigned* chunked;
+  };
+  std::vector<Rest> rest;
   for (int k = 0; k < nspecies; ++k) {
     const pic_species* s = sp + k;
     if (s->pusher == PIC_PUSHER_NONE || s->npart == 0) continue;
@@ -713,9 +738,10 @@ int pic_push_deposit(pic_ctx* c, const pic_species* sp, int32_t nspecies, const 
                           (int)tiled.size() < pic::kMaxTiledSpecies;
     if (eligible) {
       tiled.push_back(s);
-      if (b->nalive < s->npart) rest.push_back(species_tail(*s, b->nalive, c->grid.real_bytes));
+      if (b->nalive < s->npart) rest.push_back({ species_tail(*s, b->nalive, c->grid.real_bytes), nullptr });
     } else {
-      rest.push_back(*s);
+      const bool ask = exact && k < kOrderWords && s->charge != 0.0f && windows_may_pay(c, *s);
+      rest.push_back({ *s, ask ? c->jfix_bound + 1 + k : nullptr });
     }
   }
   if (!tiled.empty()) {
@@ -724,8 +750,8 @@ int pic_push_deposit(pic_ctx* c, const pic_species* sp, int32_t nspecies, const 
                                       0, -1, fjp);
     if (st != PIC_OK) return st;
   }
-  for (const pic_species& rs : rest) {
-    const pic_species* s = &rs;
+  for (const Rest& r : rest) {
+    const pic_species* s = &r.sp;
     // a species that moves but carries no charge is pushed only
     const int mode = (s->charge == 0.0f) ? pic::MODE_PUSH : pic::MODE_FUSED;
     if (mode == pic::MODE_PUSH && !write_prev) {
@@ -735,7 +761,7 @@ int pic_push_deposit(pic_ctx* c, const pic_species* sp, int32_t nspecies, const 
                      : run_pd<float>(c, s, EB, J, dt, omegaB0, dx, pic::MODE_FUSED, false, strm(stream), fjp);
     } else {
       st = is_f64(c) ? run_pd<double>(c, s, EB, J, dt, omegaB0, dx, mode, write_prev, strm(stream))
-                     : run_pd<float>(c, s, EB, J, dt, omegaB0, dx, mode, write_prev, strm(stream), fjp);
+                     : run_pd<float>(c, s, EB, J, dt, omegaB0, dx, mode, write_prev, strm(stream), fjp, r.chunked);
     }
     if (st != PIC_OK) return st;
   }

@@ -34,6 +34,8 @@ struct PDArgs {
   const unsigned* list_count = nullptr;
   // optional (FP32): deposit into the exact 64-bit accumulator instead of J
   FixedJ          fj;
+  // which of the two kernels takes the particles (BoundArgs::chunked); null: this one
+  const unsigned* chunked = nullptr;
   // elements of the EB and J arrays where these can be taken as VecField
   int             eb_count = 0, j_count = 0;
 };
@@ -221,6 +223,8 @@ __global__ void __launch_bounds__(256, (D == 2 && sizeof(real) == 4)
                                            : (VEC ? (MODE == MODE_DEPOSIT ? 3 : 2)
                                                   : (O == 3 && sizeof(real) == 4 && MODE != MODE_DEPOSIT ? 2 : 1)))
     k_push_deposit(const __grid_constant__ PDArgs<real> a) {
+  if constexpr (D == 2 && O >= 2 && sizeof(real) == 4 && MODE == MODE_FUSED && !PHOTON)
+    if (a.chunked && *a.chunked != 0u) return;
   push_deposit_all<D, O, real, MODE, PHOTON, VEC>(a);
 }
 
@@ -247,8 +251,9 @@ __global__ void __launch_bounds__(128, (D == 2 && sizeof(real) == 4) ? 6 : (O ==
 // on (2D): nodes w0 to w0 + wn - 1 per axis, ghost-free, two below the cells
 // and three above, which holds the interpolation's and the deposit's stencils
 // at every order with one cell of move. All cells that lie in the grid, or,
-// where that is more than max_nodes, those within 8 of the middle particle's;
-// none (wn = 0) when neither fits. sh: four shared ints.
+// where that is more than max_nodes, those within 8 of the middle particle's, if
+// half of the particles are there; none (wn = 0) when neither fits. sh: four shared
+// ints.
 __device__ __forceinline__ void chunk_window(const SpeciesPtrs& sp, const int* n_grid, int64_t p0,
                                              int n, int max_nodes, int* sh, int* w0, int* wn) {
   const int tid = threadIdx.x;
@@ -274,6 +279,13 @@ __device__ __forceinline__ void chunk_window(const SpeciesPtrs& sp, const int* n
   __syncthreads();
   if (cells_in_grid<2>(mid, n_grid)) {
     for (int t = 0; t < 2; ++t) {
+      if (t == 1) {
+        int near = 0;
+        for (int l = tid; l - tid < n; l += blockDim.x)
+          near += __syncthreads_count(l < n && abs(sp.i1[p0 + l] - mid[0]) <= 8 &&
+                                      abs(sp.i2[p0 + l] - mid[1]) <= 8);
+        if (2 * near < n) break;
+      }
       int64_t nodes = 1;
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
@@ -312,13 +324,14 @@ __device__ __forceinline__ void stage_window(const FieldView<real>& F, const Pus
 // atomics per particle at order 2 and by the 64-bit addresses of its 54 field
 // reads: 1.05 M cell-ordered particles, 16 per cell, took 135 us, in windows 79.
 // Particles that do not lie with the others go through the grid as before.
-constexpr int kChunkNodes = 800;  // 48 bytes each: 38 KB, four blocks per SM
 template <int O>
-__global__ void __launch_bounds__(256, O == 3 ? 3 : 4) k_push_deposit_chunk(const __grid_constant__ PDArgs<float> a, int chunk, int ls) {
+__global__ void __launch_bounds__(256, O == 3 ? 3 : 4) k_push_deposit_chunk(const __grid_constant__ PDArgs<float> a, int ls) {
+  constexpr int chunk = kChunk;
   using FA = FixedAcc<float>;
   __shared__ float    EBw[6 * kChunkNodes];
   __shared__ unsigned win[6 * kChunkNodes];
   __shared__ int      sh[4];
+  if (*a.chunked == 0u) return;
   const int64_t p0  = (int64_t)blockIdx.x * chunk;
   const int     n   = (int)(a.sp.npart - p0 < chunk ? a.sp.npart - p0 : chunk);
   const int     tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
