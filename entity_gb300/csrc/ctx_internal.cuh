@@ -70,7 +70,6 @@ struct pic_ctx {
   uint4*                                          stage_rec   = nullptr;
   unsigned*                                       stage_claim = nullptr;
   int                                             stage_slots = 0;
-  bool                                            stage_tried = false;
 };
 
 namespace pic_internal {

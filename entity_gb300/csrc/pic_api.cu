@@ -236,10 +236,10 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
     a.lane_stride     = (D == 3 && O >= 1) || ppc < 12 ? 1 : (ppc >= 24 ? 4 : 2);
   }
   cudaError_t e = cudaErrorInvalidValue;
-  if (!c->stage_tried) {
+  if (!c->stage_rec) {
     // the deposit records' buffers, once per context (its dimension, order
     // and precision fix their size); without them every particle deposits as
-    // it is pushed
+    // it is pushed, and the next call tries again
     size_t words = 0;
     int    slots = 0;
 #define PIC_RW(DD, OO) \
@@ -267,7 +267,6 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
         c->stage_slots = slots;
       }
     }
-    c->stage_tried = true;
   }
   a.st.rec    = c->stage_rec;
   a.st.claim  = c->stage_claim;
