@@ -179,6 +179,16 @@ pic_species species_tail(const pic_species& sp, int64_t first, int real_bytes) {
   return t;
 }
 
+// Clears device memory before it returns: another stream may use it next. (A stream of
+// its own: the caller's may be capturing.)
+bool clear_now(void* p, size_t bytes) {
+  cudaStream_t s = nullptr;
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return false;
+  const bool ok = cudaMemsetAsync(p, 0, bytes, s) == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+  cudaStreamDestroy(s);
+  return ok;
+}
+
 template <typename real>
 int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void* EB, void* J,
               double dt, double omegaB0, double dx, bool write_prev, cudaStream_t s,
@@ -257,7 +267,7 @@ int run_tiled(pic_ctx* c, const std::vector<const pic_species*>& sps, const void
     if (slots > 0) {
       if (cudaMalloc((void**)&c->stage_rec, sizeof(uint4) * words * (size_t)slots) != cudaSuccess ||
           cudaMalloc((void**)&c->stage_claim, sizeof(unsigned) * (size_t)slots) != cudaSuccess ||
-          cudaMemsetAsync(c->stage_claim, 0, sizeof(unsigned) * (size_t)slots, s) != cudaSuccess) {
+          !clear_now(c->stage_claim, sizeof(unsigned) * (size_t)slots)) {
         cudaGetLastError();
         if (c->stage_rec) cudaFree(c->stage_rec);
         if (c->stage_claim) cudaFree(c->stage_claim);

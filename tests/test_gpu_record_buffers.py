@@ -1,11 +1,14 @@
 """The tiled kernel's record buffers: a context that found no memory for them
-uses them once there is some."""
+uses them once there is some, and their first use from two streams at once."""
+import ctypes as C
+
 import pytest
 import torch
 
 from entity_gb300 import abi
 from entity_gb300.inputs import GridSpec, empty_field, make_species
 from entity_gb300.sim import Context
+from entity_gb300.sim import make_species as mk
 from tests.helpers import random_fields
 
 pytestmark = pytest.mark.gpu
@@ -56,3 +59,34 @@ def test_buffers_are_asked_for_again():
     assert before - torch.cuda.mem_get_info()[0] > (330 << 20)
     assert ctx.device_errors() == [0, 0, 0, 0] and ctx.wait_timeouts() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("dim,order,real", [(3, 2, torch.float32), (2, 2, torch.float32), (3, 1, torch.float64)])
+def test_first_use_from_two_streams(dim, order, real):
+    g = GridSpec(dim=dim, n=(64, 32, 32) if dim == 3 else (256, 128, 1), order=order, real=real)
+    EB = random_fields(g, 5, amp=0.1).cuda()
+    for attempt in range(4):
+        ctx, sp = _plasma(g, 6, 50)
+        ref, one = sp[0].clone(), empty_field(g, 3, "cuda")
+        L, nt = abi.load(), C.c_int64(0)
+        ps, pr = mk(sp[0], dim), mk(ref, dim)
+        assert L.pic_tile_offsets(ctx.h, C.byref(ps), None, 0, C.byref(nt), None) == abi.PIC_OK
+        cut = (0, nt.value // 2, nt.value)
+        st = [torch.cuda.Stream() for _ in range(2)]
+        Js = [empty_field(g, 3, "cuda") for _ in range(2)]
+
+        def call(s, J, lo, hi, stream):
+            assert L.pic_push_deposit_tiles(ctx.h, C.byref(s), C.c_void_p(EB.data_ptr()), C.c_void_p(J.data_ptr()),
+                                            0.3, 0.5, g.dx, lo, hi, 0, stream) == abi.PIC_OK
+        torch.cuda.synchronize()
+        for k in range(2):  # the halves of the tiles, the context's first tiled launches
+            call(ps, Js[k], cut[k], cut[k + 1], C.c_void_p(st[k].cuda_stream))
+        torch.cuda.synchronize()
+        assert ctx.device_errors() == [0, 0, 0, 0] and ctx.wait_timeouts() == 0
+        call(pr, one, 0, nt.value, None)
+        torch.cuda.synchronize()
+        assert all(torch.equal(x, y) for x, y in zip(ref.i[:dim] + ref.dx[:dim] + ref.u, sp[0].i[:dim] + sp[0].dx[:dim] + sp[0].u))
+        # float sums of the tiles' own totals, in any order: 8 tiles to an entry
+        tol = 16 * (2.0 ** -24 if real == torch.float32 else 2.0 ** -53)
+        assert float((Js[0] + Js[1] - one).abs().max()) <= tol * float(one.abs().max())
+        ctx.close()
