@@ -859,11 +859,13 @@ int pic_checkpoint_restore(pic_ctx* c, int32_t slot, pic_species* sp, int32_t ns
   if (!a || (int)a->slots.size() <= slot || !a->slots[slot].eb) return PIC_ERR_ARG;
   pic::Slot& sl = a->slots[slot];
   if ((int)sl.prt.size() != nspecies) return PIC_ERR_ARG;
+  // (before anything changes: the copies wait in a list)
+  for (int k = 0; k < nspecies; ++k)
+    if (sp[k].maxnpart > 0 && sl.npart[k] > sp[k].maxnpart) return PIC_ERR_ARG;
   cudaStream_t s = strm(stream);
   Copies copies(s);
   if (!copies.add(EB, sl.eb, a->eb_bytes)) return PIC_ERR_CUDA;
   for (int k = 0; k < nspecies; ++k) {
-    if (sp[k].maxnpart > 0 && sl.npart[k] > sp[k].maxnpart) return PIC_ERR_ARG;
     sp[k].npart = sl.npart[k];
     const char* src = (const char*)sl.prt[k];
     for (const auto& r : state_arrays(c->grid, sp[k])) {
