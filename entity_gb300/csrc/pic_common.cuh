@@ -237,7 +237,8 @@ struct VecField {
     return __ldg(p + (i + j * s1 + k * s2 + c * s3));
   }
   // the 16-byte words that hold the rows of N nodes per axis from (i, j, k) on
-  // lie within the array, for every component
+  // lie within the array, for every component (row_elements bounds the sum, for a cell
+  // of the grid)
   template <int N>
   __device__ __forceinline__ bool covers(int i, int j, int k) const {
     return i + (j + N) * s1 + (k + N) * s2 + 5 * s3 + N + 8 <= count;

@@ -42,6 +42,17 @@ enum ErrIdx {
   ERR_COUNT        = 5
 };
 
+// Elements of a float field's array where 32 bits index it by rows (VecField,
+// red_row), else 0: x1 neighbours adjacent, the array starting on 16 bytes. ext:
+// ghost-inclusive extents, s: strides of x1, x2, x3 and the component. VecField::covers
+// looks up to four rows and planes past the last cell, for a cell of the grid: the
+// sums of its indices stay below 2^31 as well.
+inline int row_elements(const void* p, const int* ext, const int64_t* s, int ncomp) {
+  if (!p || s[0] != 1 || reinterpret_cast<uintptr_t>(p) % 16 != 0) return 0;
+  const int64_t n = ext[0] + (ext[1] - 1) * s[1] + (ext[2] - 1) * s[2] + (ncomp - 1) * s[3];
+  return n + 4 * (s[1] + s[2]) + 64 <= INT32_MAX ? (int)n : 0;
+}
+
 // process-wide count of kernels this library has launched
 void note_launch();
 
