@@ -363,8 +363,8 @@ __global__ void k_fill_ghosts(GridInfo g, EdgeIter it, FieldView<real> f, int c0
 // digital filter pass in 2D: digital_filter.hpp:183-195; reads
 // src, writes dst at the active cells and their periodic ghost images
 // ---------------------------------------------------------------------------
-template <int D, typename real>
-__global__ void k_filter(GridInfo g, CellIter it, FieldView<real> src, FieldView<real> dst) {
+template <typename real>
+__global__ void k_filter2(GridInfo g, CellIter it, FieldView<real> src, FieldView<real> dst) {
   const real    INV_4 = 0.25, INV_8 = 0.125, INV_16 = 0.0625;
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < it.count; t += stride) {
@@ -374,7 +374,6 @@ __global__ void k_filter(GridInfo g, CellIter it, FieldView<real> src, FieldView
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
 #define b(x, y, z) src.p[src.idx(x, y, z, c)]
-      static_assert(D == 2, "the 3D passes are below");
       nv[c] = INV_4 * b(i1, i2, 0) +
               INV_8 * (b(i1 - 1, i2, 0) + b(i1 + 1, i2, 0) + b(i1, i2 - 1, 0) + b(i1, i2 + 1, 0)) +
               INV_16 * (b(i1 - 1, i2 - 1, 0) + b(i1 + 1, i2 + 1, 0) + b(i1 - 1, i2 + 1, 0) +
@@ -383,7 +382,7 @@ __global__ void k_filter(GridInfo g, CellIter it, FieldView<real> src, FieldView
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) dst.p[dst.idx(i1, i2, i3, c)] = nv[c];
-    for_images<D>(g, i1, i2, i3, [&](int a, int bb, int e) {
+    for_images<2>(g, i1, i2, i3, [&](int a, int bb, int e) {
 #pragma unroll
       for (int c = 0; c < 3; ++c) dst.p[dst.idx(a, bb, e, c)] = nv[c];
     });
@@ -729,7 +728,7 @@ cudaError_t launch_filter(const GridInfo& g, FieldView<real> J, FieldView<real> 
     // ping-pong: every ghost cell is an image and is rewritten each pass
     FieldView<real> a = J, b = buff;
     for (int p = 0; p < npasses; ++p) {
-      if (g.dim == 2) PIC_KL(k_filter<2, real><<<gr, 256, 0, s>>>(g, it, a, b));
+      if (g.dim == 2) PIC_KL(k_filter2<real><<<gr, 256, 0, s>>>(g, it, a, b));
       else            filter3(g, a, b, s);
       FieldView<real> t = a;
       a                 = b;
@@ -740,7 +739,7 @@ cudaError_t launch_filter(const GridInfo& g, FieldView<real> J, FieldView<real> 
     // reference order: buff <- J (incl. non-periodic ghosts), filter, fill
     for (int p = 0; p < npasses; ++p) {
       PIC_KL(k_copy3<real><<<grc, 256, 0, s>>>(g, J, buff));
-      if (g.dim == 2) PIC_KL(k_filter<2, real><<<gr, 256, 0, s>>>(g, it, buff, J));
+      if (g.dim == 2) PIC_KL(k_filter2<real><<<gr, 256, 0, s>>>(g, it, buff, J));
       else            filter3(g, buff, J, s);
     }
   }

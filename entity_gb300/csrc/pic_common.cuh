@@ -233,9 +233,6 @@ struct VecField {
   int                   s1, s2, s3, count;  // count: elements of the array
   __device__ __forceinline__ VecField(const FieldView<float>& f, int n)
       : p(f.p), s1((int)f.s1), s2((int)f.s2), s3((int)f.s3), count(n) {}
-  __device__ __forceinline__ float ld(int i, int j, int k, int c) const {
-    return __ldg(p + (i + j * s1 + k * s2 + c * s3));
-  }
   // the 16-byte words that hold the rows of N nodes per axis from (i, j, k) on
   // lie within the array, for every component (row_elements bounds the sum, for a cell
   // of the grid)
@@ -685,7 +682,7 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
                                                       int ng, const int* ext, Add&& add) {
   constexpr bool UNMOVED = BOX == BOX_UNMOVED;
   static_assert(BOX == BOX_ANY || O >= 1, "the zigzag deposit has no support box");
-  static_assert(FACTORED || BOX != BOX_UNMOVED, "the reference's form takes any extent");
+  static_assert(FACTORED || BOX == BOX_ANY, "the reference's form takes any extent");
   const real ONE = 1, HALF = 0.5, INV_2 = 0.5;
   if constexpr (O == 0) {
     if (ext) {
@@ -773,11 +770,9 @@ __device__ __forceinline__ bool deposit_with_velocity(const Prtl<real>& q, const
     constexpr real THIRD = K<real>::THIRD;
     const real     Q     = coeff * inv_dt;
     if constexpr (!FACTORED) {
-      // the add of an entry inside the particle's extent; in a full box an
-      // entry outside adds an exact zero
+      // the add of an entry inside the particle's extent
       auto put = [&](bool in, int i, int j, int k, int c, real v) {
-        if constexpr (BOX == BOX_FULL) add(i, j, k, c, in ? v : (real)0);
-        else if (in) add(i, j, k, c, v);
+        if (in) add(i, j, k, c, v);
       };
       const int  d1 = imax[0] - imin[0], d2 = imax[1] - imin[1];
       const int  i0 = imin[0] + ng, j0 = imin[1] + ng;
