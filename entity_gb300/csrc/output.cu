@@ -19,6 +19,7 @@
 // like the reference's ScatterView on CUDA.
 #include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "ctx_internal.cuh"
 
@@ -159,13 +160,15 @@ template <int T, int C, int N>
 struct MomBlock {
   static constexpr int THREADS = T, CHUNK = C, NODES = N;
 };
+using MomDense = MomBlock<512, 4096, 4096>;
 using MomLarge = MomBlock<512, 2048, 4352>;
 using MomSmall = MomBlock<256, 512, 2560>;
+using MomWide  = MomBlock<256, 512, 3840>;  // orders 5 and 6
 
 // Window sums in fixed point. A contribution v, |v| <= 2^18, is split into
 // h + l 2^-19 (two words) or h + m 2^-19 + l 2^-38 (three), integers of at most 2^18
 // each, all but the last exact, and each is added to a 32-bit word: a chunk's additions
-// (2^11 at most) stay within 2^29. The integers come by adding 1.5 * 2^23, whose
+// (2^12 at most) stay within 2^30. The integers come by adding 1.5 * 2^23, whose
 // sum's low mantissa bits they are.
 constexpr int kMomTop = 18, kMomStep = 19;
 template <int WORDS>
@@ -180,11 +183,19 @@ __device__ __forceinline__ void moment_add(int* w, int plane, float v) {
     atomicAdd(w + k * plane, __float_as_int(t) - 0x4B400000);
   }
 }
-// the sum of a node, in units of 2^-kMomStep
+// The sum of a node times 2^e. Two words: one conversion and two exact scalings (2^e
+// itself may be no normal float), because FP64 runs at 1/64 of the FP32 rate: in
+// double the flush took a twelfth of the kernel.
 template <int WORDS>
-__device__ __forceinline__ double moment_total(const int* w, int plane) {
-  const double t = (double)((long long)w[0] * (1 << kMomStep) + w[plane]);
-  return WORDS == 2 ? t : t + (double)w[(WORDS - 1) * plane] * (1.0 / (1 << kMomStep));
+__device__ __forceinline__ float moment_total(const int* w, int plane, int e) {
+  const long long t = (long long)w[0] * (1 << kMomStep) + w[plane];
+  if constexpr (WORDS == 2) {
+    const int a = (e - kMomStep) / 2;
+    return __ll2float_rn(t) * __int_as_float((127 + a) << 23) *
+           __int_as_float((127 + e - kMomStep - a) << 23);
+  } else {
+    return (float)ldexp((double)t + (double)w[2 * plane] * (1.0 / (1 << kMomStep)), e - kMomStep);
+  }
 }
 // the block's largest coefficient over the largest of a cell, at most, for two words
 // and for three
@@ -282,8 +293,9 @@ constexpr size_t moment_smem() {
 // A particle makes (2 W + 1)^D additions, which bound the kernel. 16.8 M
 // sorted particles at order 2 took 1.64 ms with global atomics, which meet in
 // a few L2 lines, 1.05 ms in the window in their own order (the lanes of one
-// cell meet in its words, eight wavefronts an atomic), and 0.45 ms queued by
-// bank, a warp's 32 lanes adding in 32 banks.
+// cell meet in its words, eight wavefronts an atomic), and 0.43 ms queued by
+// bank, a warp's 32 lanes adding in 32 banks (with sums of 30 bits; 7.1 M took 191
+// us with those, 203 us with these).
 template <int D, int ORDER, typename B>
 __global__ void __launch_bounds__(B::THREADS) k_output_moment(MomArgs<float> a,
                                                               unsigned long long* err) {
@@ -462,10 +474,10 @@ __global__ void __launch_bounds__(B::THREADS) k_output_moment(MomArgs<float> a,
   else
     deposit([&](int e, real coeff, real sh) { moment_add<3>(win + e, nodes, (coeff * scale) * sh); });
   __syncthreads();
-  const double unscale = ldexp(1.0, ex - kMomTop - kMomStep);
   for (int e = tid; e < nodes; e += kMomThreads) {
-    const double v = words == 2 ? moment_total<2>(win + e, nodes) : moment_total<3>(win + e, nodes);
-    if (v != 0.0) on_grid(e, (real)(v * unscale));
+    const real v = words == 2 ? moment_total<2>(win + e, nodes, ex - kMomTop)
+                              : moment_total<3>(win + e, nodes, ex - kMomTop);
+    if (v != (real)0) on_grid(e, v);
   }
 }
 
@@ -487,9 +499,22 @@ cudaError_t launch_moment(const MomArgs<real>& a, unsigned long long* err, cudaS
   // same, a 3D block of 512 threads had an SM to itself: 27,648 particles at order 2
   // took 157 us there, 13 us so, 7.1 M 1.96 and 1.81 ms, 480,000 in 2D 88 and 68 us
   if constexpr (sizeof(real) == 4) {
-    return a.sp.npart / MomLarge::CHUNK >= 3 * pic::sm_count()
-             ? launch_moment_window<D, ORDER, MomLarge>(a, err, s)
-             : launch_moment_window<D, ORDER, MomSmall>(a, err, s);
+    // Three large blocks per SM at least, else small ones; the largest in 3D from 8
+    // particles per cell on, where their windows still hold most chunks. Small,
+    // 2048 and 4096 particles, us at order 2: 27,648 at 2 per cell 9, 19 and 31; 1.0 M at
+    // 4 per cell 41, 37 and 45; 7.1 M at 8 per cell 258, 222 and 203 (order 3 746, 607
+    // and 583); 6.5 M in 2D 147, 114 and 142.
+    // Orders 5 and 6, seldom used and long to compile, have small ones with room for
+    // their wider windows at every size.
+    if constexpr (ORDER <= 4) {
+      if (a.sp.npart / MomLarge::CHUNK >= 3 * pic::sm_count()) {
+        if constexpr (D == 3)
+          if (a.sp.npart >= 8 * (int64_t)a.n[0] * a.n[1] * a.n[2])
+            return launch_moment_window<D, ORDER, MomDense>(a, err, s);
+        return launch_moment_window<D, ORDER, MomLarge>(a, err, s);
+      }
+    }
+    return launch_moment_window<D, ORDER, std::conditional_t<ORDER <= 4, MomSmall, MomWide>>(a, err, s);
   } else {
     PIC_KL(k_output_moment_direct<D, ORDER, real><<<blocks_for(a.sp.npart), 256, 0, s>>>(a, err));
     return cudaGetLastError();

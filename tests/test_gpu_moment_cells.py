@@ -126,3 +126,19 @@ def test_layouts(dim, layout, weight):
     # random order about 5 particles a cell, each touching 27 nodes, 200 at the most
     n = 20 + {"cells": 27, "clump": 27 + 40, "random": 200, "cell": 81}[layout]
     _check(g, s, [(N, 0, 0, 0, SPLINE), (N, 0, 0, 2, SPLINE), (T, 0, 1, 1, SPLINE), (V, 2, 0, 2, CONST)], n)
+
+
+# the lines between the block sizes: three blocks of 2048 per SM of 152, 8 particles per cell
+@pytest.mark.parametrize("dim,n,count", [
+    (3, (40, 40, 73), 3 * 152 * 2048 - 1), (3, (40, 40, 73), 3 * 152 * 2048 + 2047), (3, (48, 48, 50), 8 * 48 * 48 * 50 - 1),
+    (3, (48, 48, 50), 8 * 48 * 48 * 50 + 4097), (2, (320, 300, 1), 3 * 152 * 2048 + 1), (2, (70, 61, 1), 513), (3, (20, 18, 12), 33)])
+@pytest.mark.parametrize("layout", ["cells", "clump"])
+def test_block_sizes(dim, n, count, layout, monkeypatch):
+    monkeypatch.setitem(globals(), "COUNT", count)
+    g = GridSpec(dim=dim, n=n, order=2, real=torch.float32)
+    s, rand = _particles(g, layout, 11)
+    s.w = 0.5 + rand()
+    # in these grids a chunk's cells may not fit a window: then every particle of the
+    # 27 cells (9 to 30 each) adds by itself
+    per = -(-count // g.ncells()) + 12
+    _check(g, s, [(N, 0, 0, 2, SPLINE), (T, 1, 2, 2, CONST)], 20 + 27 * per)
