@@ -67,26 +67,27 @@ def test_first_use_from_two_streams(dim, order, real):
     EB = random_fields(g, 5, amp=0.1).cuda()
     for attempt in range(4):
         ctx, sp = _plasma(g, 6, 50)
-        ref, one = sp[0].clone(), empty_field(g, 3, "cuda")
+        ref = [s.clone() for s in sp]
+        Js = [empty_field(g, 3, "cuda") for _ in range(4)]
         L, nt = abi.load(), C.c_int64(0)
-        ps, pr = mk(sp[0], dim), mk(ref, dim)
-        assert L.pic_tile_offsets(ctx.h, C.byref(ps), None, 0, C.byref(nt), None) == abi.PIC_OK
-        cut = (0, nt.value // 2, nt.value)
+        assert L.pic_tile_offsets(ctx.h, C.byref(mk(sp[0], dim)), None, 0, C.byref(nt), None) == abi.PIC_OK
         st = [torch.cuda.Stream() for _ in range(2)]
-        Js = [empty_field(g, 3, "cuda") for _ in range(2)]
 
-        def call(s, J, lo, hi, stream):
-            assert L.pic_push_deposit_tiles(ctx.h, C.byref(s), C.c_void_p(EB.data_ptr()), C.c_void_p(J.data_ptr()),
-                                            0.3, 0.5, g.dx, lo, hi, 0, stream) == abi.PIC_OK
+        def call(s, J, stream):
+            assert L.pic_push_deposit_tiles(ctx.h, C.byref(mk(s, dim)), C.c_void_p(EB.data_ptr()),
+                                            C.c_void_p(J.data_ptr()), 0.3, 0.5, g.dx, 0, nt.value, 0, stream) == abi.PIC_OK
         torch.cuda.synchronize()
-        for k in range(2):  # the halves of the tiles, the context's first tiled launches
-            call(ps, Js[k], cut[k], cut[k + 1], C.c_void_p(st[k].cuda_stream))
+        for k in range(2):  # a species to a stream: the context's first tiled launches
+            call(sp[k], Js[k], C.c_void_p(st[k].cuda_stream))
         torch.cuda.synchronize()
         assert ctx.device_errors() == [0, 0, 0, 0] and ctx.wait_timeouts() == 0
-        call(pr, one, 0, nt.value, None)
+        for k in range(2):
+            call(ref[k], Js[2 + k], None)
         torch.cuda.synchronize()
-        assert all(torch.equal(x, y) for x, y in zip(ref.i[:dim] + ref.dx[:dim] + ref.u, sp[0].i[:dim] + sp[0].dx[:dim] + sp[0].u))
         # float sums of the tiles' own totals, in any order: 8 tiles to an entry
         tol = 16 * (2.0 ** -24 if real == torch.float32 else 2.0 ** -53)
-        assert float((Js[0] + Js[1] - one).abs().max()) <= tol * float(one.abs().max())
+        for k in range(2):
+            a, b = ref[k], sp[k]
+            assert all(torch.equal(x, y) for x, y in zip(a.i[:dim] + a.dx[:dim] + a.u, b.i[:dim] + b.dx[:dim] + b.u))
+            assert float((Js[k] - Js[2 + k]).abs().max()) <= tol * float(Js[2 + k].abs().max())
         ctx.close()
