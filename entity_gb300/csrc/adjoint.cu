@@ -528,7 +528,10 @@ cudaError_t launch_push_deposit_adjoint(int order, const AdjArgs<real>& args, cu
   AdjArgs<real> a = args;
   const bool    rows = packed(a.EB, 6) && packed(a.lam, 6) && packed(a.lamJ, 3) &&
                     (uintptr_t)a.lam.p % 16 == 0;
-  if (rows) a.lam_count = (int)(a.pc.ext[0] + (a.pc.ext[1] - 1) * a.lam.s1 + 5 * a.lam.s3);
+  // (no elements for the vector additions where the array has gaps)
+  const int     ext[3] = { a.pc.ext[0], a.pc.ext[1], 1 };
+  const int64_t ls[4]  = { a.lam.s0, a.lam.s1, a.lam.s2, a.lam.s3 };
+  if (rows && no_gaps(ext, ls)) a.lam_count = (int)(6 * ls[3]);
 #define PIC_ADJ(OO)                                                                            \
   case OO:                                                                                     \
     if (rows) PIC_KL(k_push_deposit_adjoint<OO, real, RowView><<<g, 256, 0, s>>>(a));          \

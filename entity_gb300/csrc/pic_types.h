@@ -53,6 +53,14 @@ inline int row_elements(const void* p, const int* ext, const int64_t* s, int nco
   return n + 4 * (s[1] + s[2]) + 64 <= INT32_MAX ? (int)n : 0;
 }
 
+// Whether the array has no gaps between its elements. Sums are added by 16-byte words
+// (red_row) only then: a word's other floats get zeros, which would flush what lies
+// in a gap.
+inline bool no_gaps(const int* ext, const int64_t* s) {
+  return s[0] == 1 && s[1] == ext[0] && (ext[2] == 1 || s[2] == (int64_t)ext[0] * ext[1]) &&
+         s[3] == (int64_t)ext[0] * ext[1] * ext[2];
+}
+
 // process-wide count of kernels this library has launched
 void note_launch();
 
