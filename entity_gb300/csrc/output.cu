@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(B::THREADS) k_output_moment(MomArgs<float> a,
   if (lane == 0) atomicMin(&s_min, least);
   __syncthreads();
   const float top = __uint_as_float(s_max), low = __uint_as_float(s_min);
-  if (top == 0.f) return;
+  if (top == 0.f && !s_bad) return;
   const int words = s_bad || top < 0x1p-108f ? 0
                     : top <= kMomRange2 * low ? 2
                     : top <= kMomRange3 * low && 3 * nodes <= 2 * B::NODES ? 3 : 0;

@@ -142,3 +142,34 @@ def test_block_sizes(dim, n, count, layout, monkeypatch):
     # 27 cells (9 to 30 each) adds by itself
     per = -(-count // g.ncells()) + 12
     _check(g, s, [(N, 0, 0, 2, SPLINE), (T, 1, 2, 2, CONST)], 20 + 27 * per)
+
+
+@pytest.mark.parametrize("which", ["one", "all"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_weights_that_are_not_finite(which, value):
+    """They reach the nodes of their particles, and no others."""
+    g = GridSpec(dim=3, n=(16, 16, 256), order=2, real=torch.float32)
+    s, _ = _particles(g, "cells", 13)
+    s.tag[:] = 1
+    s.w[:] = 1.0
+    at = slice(5000, 5001) if which == "one" else slice(0, 3 * 4096)
+    if which == "all":
+        s.w[at] = 0.0
+    s.w[at] = value
+    ctx = Context(g)
+    p = abi.PicMomentParams()
+    p.id, p.order, p.smoothing, p.use_weights, p.inv_n0, p.dx = N, 1, CONST, 1, 0.5, 0.75
+    buf = empty_field(g, 6, "cuda")
+    ctx.output_moment([s], p, buf, 0)
+    torch.cuda.synchronize()
+    hit = torch.zeros(buf[0].numel(), dtype=torch.bool, device="cuda")
+    for k in range(27):
+        d = [k % 3 - 1, k // 3 % 3 - 1, k // 9 - 1]
+        flat = 0
+        for a in reversed(range(3)):
+            flat = flat * g.ext[a] + s.i[a][at].long() + d[a] + g.ng
+        hit[flat] = True
+    assert torch.equal(~torch.isfinite(buf[0]).reshape(-1), hit)
+    assert float(buf[0][torch.isfinite(buf[0])].abs().max()) > 0
+    ctx.close()
+
