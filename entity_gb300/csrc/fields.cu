@@ -516,8 +516,11 @@ __global__ void __launch_bounds__(256) k_filter3_staged(GridInfo g, FieldView<do
                 TRIPS = (NS + 255) / 256;
   __shared__ double sm[3][SZ][SY][SX];
   const int ng = g.ng;
-  // first active cell of the block, ghost-inclusive
-  const int x0 = ng + blockIdx.x * kFltX, y0 = ng + blockIdx.y * kFltY, i3 = ng + blockIdx.z;
+  // first active cell of the block, ghost-inclusive (a plane per block can be more
+  // planes than a grid's y and z hold)
+  const int bx = (g.n[0] + kFltX - 1) / kFltX, by = (g.n[1] + kFltY - 1) / kFltY;
+  const int x0 = ng + (int)(blockIdx.x % bx) * kFltX, y0 = ng + (int)(blockIdx.x / bx % by) * kFltY,
+            i3 = ng + (int)(blockIdx.x / bx / by);
   const int ex = g.n[0] + 2 * ng, ey = g.n[1] + 2 * ng;
   // a fixed trip count, unrolled: every thread's loads are in flight together
   double v[TRIPS];
@@ -563,7 +566,7 @@ void filter3(const GridInfo& g, FieldView<float> a, FieldView<float> b, cudaStre
   PIC_KL(k_filter3_march<<<dim3(bx, by, (g.n[2] + zlen - 1) / zlen), 256, 0, s>>>(g, a, b, zlen));
 }
 void filter3(const GridInfo& g, FieldView<double> a, FieldView<double> b, cudaStream_t s) {
-  const dim3 blocks((g.n[0] + kFltX - 1) / kFltX, (g.n[1] + kFltY - 1) / kFltY, g.n[2]);
+  const unsigned blocks = (unsigned)((g.n[0] + kFltX - 1) / kFltX) * ((g.n[1] + kFltY - 1) / kFltY) * g.n[2];
   PIC_KL(k_filter3_staged<<<blocks, 256, 0, s>>>(g, a, b));
 }
 
