@@ -639,7 +639,9 @@ int pic_deposit(pic_ctx* c, const pic_species* sp, int32_t nspecies, void* J, do
 // particles and few per cell go without: the kernel that leaves at once and the look at
 // the order take 5 us. In random order windows lose (900^2, 32 per cell, order 2: 5.8
 // ms instead of 4.5).
-static bool windows_may_pay(const pic_ctx* c, const pic_species& sp) {
+static bool windows_may_pay(pic_ctx* c, const pic_species& sp) {
+  const SpeciesBins* b = find_bins(c, sp.index, false);
+  if (b && b->valid && b->npart == sp.npart) return false;  // the tiled kernel's
   return c->grid.dim == 2 && c->grid.order >= 2 && sp.pusher != PIC_PUSHER_PHOTON &&
          sp.npart >= (1 << 19) && sp.npart >= 8 * (int64_t)c->grid.n[0] * c->grid.n[1];
 }
